@@ -44,7 +44,7 @@ def _rc(rc: int, what: str):
 def available(space: str = "serial") -> bool:
     """True when the library is built, or can be built because the reference
     sources are present on this machine."""
-    return os.path.exists(_LIBS[space]) or os.path.isdir(_REF_SRC)
+    return os.path.exists(_LIBS[space]) or os.path.exists(os.path.join(_REF_SRC, "src", "jet.cpp"))
 
 
 def build() -> None:
@@ -56,7 +56,7 @@ def lib(space: str = "serial"):
     if space not in _loaded:
         path = _LIBS[space]
         if not os.path.exists(path):
-            if not os.path.isdir(_REF_SRC):
+            if not os.path.exists(os.path.join(_REF_SRC, "src", "jet.cpp")):
                 raise RuntimeError("%s is not built and the reference sources are absent" % path)
             build()
         lib_ = ctypes.CDLL(path)
