@@ -177,6 +177,10 @@ def run_reference(args, wl, rank):
     if rank != 0:
         return
     oracle, ref = _oracle_mods()
+    if not ref.available("host"):
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's sources are absent and its CPU build "
+                          "(oracle/_ref) was not made"}), flush=True)
+        return
     jet = load_pkg()
     g = wl["make"](jet.graphs, "cpu")
     og = oracle.G.from_csr(g)
@@ -845,7 +849,9 @@ def main():
     e2e_value = ws * len(e2e_times) / sum(e2e_times) if e2e_times else None
     stage("e2e done")
     cpu_cores = 0
-    if ws == 1 and not args.no_cpu_baseline:
+    # the CPU baselines are the reference's own host build; without it they are left out
+    have_ref = ws == 1 and not args.no_cpu_baseline and _oracle_mods()[1].available("host")
+    if have_ref:
         cpu_cores = _oracle_mods()[1].concurrency("host")
     batched = run_batched(jet, dev, args.batched, args.workers, ws, rank, dist, cpu_cores) if args.batched > 0 else None
     stage("batched done")
@@ -894,7 +900,7 @@ def main():
             roof["finest_table_build"] = tb
     stage("power-law done")
     cpu_base = None
-    if ws == 1 and not args.no_cpu_baseline:
+    if have_ref:
         dt, ocut, oimb = reference_partition(host_graph(g), wl, 1)
         stage("CPU baseline done")
     if powerlaw is not None and args.check_scale > 0:
