@@ -902,15 +902,15 @@ def main():
     cpu_base = None
     if have_ref:
         dt, ocut, oimb = reference_partition(host_graph(g), wl, 1)
+        cpu_base = {"value": 1.0 / dt, "unit": "graphs/s", "cores": cpu_cores, "kind": "reference",
+                    "sample": "one full partition of the same graph by the reference's jet_host path on %d OpenMP "
+                              "threads, cut %d" % (cpu_cores, ocut)}
         stage("CPU baseline done")
     if powerlaw is not None and args.check_scale > 0:
         # last, alone: the oracle's partition of a smaller power-law graph in
         # a child process (its host work would disturb the other legs)
         powerlaw["oracle_check"] = finish_oracle_check(jet, start_oracle_check(jet, dev, args.check_scale))
         stage("oracle check done")
-        cpu_base = {"value": 1.0 / dt, "unit": "graphs/s", "cores": cpu_cores, "kind": "reference",
-                    "sample": "one full partition of the same graph by the reference's jet_host path on %d OpenMP "
-                              "threads, cut %d" % (cpu_cores, ocut)}
     sorted_t = sorted(times)
     line = {
         "metric": "graphs/sec", "value": value, "unit": "graphs/s", "n_gpus": ws, "steps": args.steps,
