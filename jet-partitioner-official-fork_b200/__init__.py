@@ -163,7 +163,13 @@ def _ptr(t: Optional[torch.Tensor]):
 
 
 def _stream_ptr(stream=None):
+    """The stream a call runs on.  For torch's default stream (handle 0) the
+    library uses a non-blocking stream of its own, which nothing orders after
+    the default stream's work: what is still writing the inputs there is waited
+    for first."""
     s = stream if stream is not None else torch.cuda.current_stream()
+    if s.cuda_stream == 0:
+        s.synchronize()
     return ctypes.c_void_p(s.cuda_stream)
 
 

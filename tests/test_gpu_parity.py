@@ -614,3 +614,22 @@ def test_rmat24_k256_full_size_equals_oracle_fixture(jet, graphs):
     assert cut == want["cut"]
     assert hashlib.sha256(host(part).astype(np.int32).tobytes()).hexdigest() == want["part_sha256"]
     assert exp.imb_ratio <= 1.10 + 1e-12
+
+
+def test_inputs_still_being_written_on_the_default_stream(jet, graphs):
+    """A call on torch's default stream waits for the work queued there: the
+    graph's arrays are filled behind a long kernel, with no synchronisation
+    before the call."""
+    g = make(graphs, "grid2d", "i32").to("cuda")
+    cfg = jet.config_t(coarsening_alg=1, num_parts=8, max_imb_ratio=1.03)
+    want, cut, _ = jet.partition(cfg, g, seed=5)
+    late = graphs.CSRGraph(g.n, torch.zeros_like(g.row), torch.zeros_like(g.adj), torch.ones_like(g.val),
+                           torch.ones_like(g.vw), g.uniform, g.tier)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(50_000_000)  # about 25 ms
+    late.row.copy_(g.row)
+    late.adj.copy_(g.adj)
+    late.val.copy_(g.val)
+    late.vw.copy_(g.vw)
+    got, got_cut, _ = jet.partition(cfg, late, seed=5)
+    assert got_cut == cut and torch.equal(got, want)
