@@ -382,12 +382,17 @@ __global__ void __launch_bounds__(1024) k_pick_match_hub(GView<O, E, W> g, const
     }
 }
 
+// The vertex hash of the caller's ordinal width: 8-byte keys when the ids came
+// as 64-bit ones (`h64`), whatever width they are held in here.
+template <class O>
+__device__ __forceinline__ uint32_t id_hash(O x, int h64) { return h64 ? pod_hash((int64_t)x) : pod_hash(x); }
+
 // Commit rounds, src/heuristics.hpp:462-501.  Part 1 marks inactive
 // vertices; in part 2 an inactive v goes to the first active proposer in
 // index order (what the reference's in-order pass yields), found with
 // atomicMin so the outcome does not depend on thread timing.
 template <class O>
-__global__ void k_commit1(O n, const O* perm, const O* perm_len, const O* hn, O* vcmap, O* winner, int r) {
+__global__ void k_commit1(O n, const O* perm, const O* perm_len, const O* hn, O* vcmap, O* winner, int r, int h64) {
     const O MAXV = ord_max<O>();
     O len = perm ? *perm_len : n;
     for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < len; x += (int64_t)gridDim.x * blockDim.x) {
@@ -395,7 +400,7 @@ __global__ void k_commit1(O n, const O* perm, const O* perm_len, const O* hn, O*
         winner[u] = MAXV;
         O v = hn[u];
         if (v == MAXV || vcmap[u] != MAXV) continue;
-        bool cond = r > 0 ? (pod_hash((O)(u + r)) < pod_hash((O)(v + r))) : (u < v);
+        bool cond = r > 0 ? (id_hash<O>((O)(u + r), h64) < id_hash<O>((O)(v + r), h64)) : (u < v);
         if (!cond) vcmap[u] = MAXV - 1;
     }
 }
@@ -494,12 +499,12 @@ __global__ void k_leaf_hash(GView<O, E, W> g, const O* list, O cnt, O* hashes) {
 // Order-free adjacency digest sum(h^2 + h), h = pod_hash(neighbour)
 // (src/heuristics.hpp:580-594).  One warp per vertex; one CTA per hub.
 template <class O, class E, class W>
-__global__ void __launch_bounds__(BLOCK) k_twin_hash(GView<O, E, W> g, const O* list, O cnt, uint64_t* hashes) {
+__global__ void __launch_bounds__(BLOCK) k_twin_hash(GView<O, E, W> g, const O* list, O cnt, uint64_t* hashes, int h64) {
 #define TWIN_BODY(x, in, lane)                                                              \
     {                                                                                       \
         uint64_t h = 0; O u = 0; E s = 0, e = 0;                                            \
         if (in) { u = list[x]; s = g.row[u]; e = g.row[u + 1]; if (e - s > HUB_DEG) e = s; } \
-        for (E j = s + lane; j < e; j += 32) { uint64_t y = pod_hash(g.adj[j]); h += y * y + y; } \
+        for (E j = s + lane; j < e; j += 32) { uint64_t y = id_hash<O>(g.adj[j], h64); h += y * y + y; } \
         h = group_sum<uint64_t>(h, 32);                                                     \
         if (in && lane == 0 && g.row[u + 1] - s <= HUB_DEG) hashes[x] = h;                  \
     }
@@ -511,14 +516,14 @@ __global__ void __launch_bounds__(BLOCK) k_twin_hash(GView<O, E, W> g, const O* 
 // position pos[u].
 template <class O, class E, class W>
 __global__ void __launch_bounds__(1024) k_twin_hash_hub(GView<O, E, W> g, const O* hub_list, O n_hub, const O* vcmap,
-                                                        const O* pos, uint64_t* hashes) {
+                                                        const O* pos, uint64_t* hashes, int h64) {
     __shared__ uint64_t part[32];
     for (O x = blockIdx.x; x < n_hub; x += gridDim.x) {
         O u = hub_list[x];
         if (vcmap[u] != ord_max<O>()) continue;
         E s = g.row[u], e = g.row[u + 1];
         uint64_t h = 0;
-        for (E j = s + threadIdx.x; j < e; j += blockDim.x) { uint64_t y = pod_hash(g.adj[j]); h += y * y + y; }
+        for (E j = s + threadIdx.x; j < e; j += blockDim.x) { uint64_t y = id_hash<O>(g.adj[j], h64); h += y * y + y; }
         h = group_sum<uint64_t>(h, 32);
         if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = h;
         __syncthreads();

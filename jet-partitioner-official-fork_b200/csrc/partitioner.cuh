@@ -36,6 +36,7 @@ struct Engine {
     int64_t* hscal = nullptr;  // pinned mirror
     IterResult* hres = nullptr;
     int slot0 = -1;
+    int hash64 = 0;  // the caller's ids were 64-bit ones (id_hash)
 
     // side streams for the independent contraction bins of large levels
     // (made on first use), with the fork and join events
@@ -210,7 +211,7 @@ struct Engine {
         while (len > 0) {
             unsigned grid = grid_persistent(len, 16);
             for (int r = 0; r < 4; r++) {
-                k_commit1<O><<<grid, BLOCK, 0, s>>>(n, cur, cur_len, hn.p, vcmap, winner.p, r); count_launch();
+                k_commit1<O><<<grid, BLOCK, 0, s>>>(n, cur, cur_len, hn.p, vcmap, winner.p, r, hash64); count_launch();
                 k_commit2a<O><<<grid, BLOCK, 0, s>>>(n, cur, cur_len, hn.p, vcmap, winner.p); count_launch();
                 k_commit2<O><<<grid, BLOCK, 0, s>>>(n, cur, cur_len, hn.p, vcmap, winner.p); count_launch();
                 k_commit3<O><<<grid, BLOCK, 0, s>>>(n, cur, cur_len, vcmap); count_launch();
@@ -309,11 +310,11 @@ struct Engine {
             O cnt = unmatched_list(L, vcmap, 0, list, &pos);
             if (cnt > 0) {
                 DBuf<uint64_t> hs(cnt, s);
-                k_twin_hash<O, E, W><<<grid_persistent((int64_t)cnt * 32, 16), BLOCK, 0, s>>>(g, list.p, cnt, hs.p); count_launch();
+                k_twin_hash<O, E, W><<<grid_persistent((int64_t)cnt * 32, 16), BLOCK, 0, s>>>(g, list.p, cnt, hs.p, hash64); count_launch();
                 JET_LAUNCH_CHECK();
                 if (L.n_hub > 0) {
                     k_twin_hash_hub<O, E, W><<<grid_for(L.n_hub, 1) < 4096 ? grid_for(L.n_hub, 1) : 4096, 1024, 0, s>>>(
-                        g, L.hub_list.p, L.n_hub, vcmap, pos.p, hs.p); count_launch();
+                        g, L.hub_list.p, L.n_hub, vcmap, pos.p, hs.p, hash64); count_launch();
                     JET_LAUNCH_CHECK();
                 }
                 match_hash<uint64_t>(list.p, hs.p, cnt, (uint64_t)0, (uint64_t)0, 64, vcmap);

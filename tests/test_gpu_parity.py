@@ -633,3 +633,57 @@ def test_inputs_still_being_written_on_the_default_stream(jet, graphs):
     late.vw.copy_(g.vw)
     got, got_cut, _ = jet.partition(cfg, late, seed=5)
     assert got_cut == cut and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("alg", [0, 1, 2])
+@pytest.mark.parametrize("tier", ["big", "biggest"])
+@pytest.mark.parametrize("kind,k", [("grid2d", 7), ("rgg", 16), ("rmat", 16), ("star", 8), ("dense", 300)])
+def test_64_bit_tiers_in_32_bits(jet, graphs, tier, kind, k, alg, tmp_path, monkeypatch):
+    """A 64-bit-tier graph whose sums fit 32 bits is partitioned in 32 bits;
+    a run that dumps its hierarchy keeps the tier's own types.  Both give the
+    same partition, with vertex weights and from host memory too."""
+    monkeypatch.chdir(tmp_path)
+    g = make(graphs, kind, tier)
+    g.vw = torch.randint(1, 6, (g.n,), generator=torch.Generator().manual_seed(3)).to(g.vw.dtype)
+    fn = {"big": jet.partition_big, "biggest": jet.partition_biggest}[tier]
+    hfn = {"big": jet.partition_host_big, "biggest": jet.partition_host_biggest}[tier]
+    for ultra in (False, True):
+        a = dict(coarsening_alg=alg, num_parts=k, max_imb_ratio=1.05, ultra_settings=ultra)
+        part, cut, _ = fn(jet.config_t(**a), g.to("cuda"), seed=3)
+        want, wcut, _ = fn(jet.config_t(dump_coarse=True, **a), g.to("cuda"), seed=3)
+        assert cut == wcut and torch.equal(part, want)
+        hpart, hcut, _ = hfn(jet.config_t(verbose=True, **a), g, seed=3)
+        assert hcut == wcut and torch.equal(hpart, want.cpu())
+
+
+@pytest.mark.parametrize("tier", ["big", "biggest"])
+@pytest.mark.parametrize("which,off", [("edges", -2), ("edges", 0), ("edges", 4), ("vertices", -1), ("vertices", 0),
+                                       ("single", 0)])
+def test_32_bit_rule_at_its_edges(jet, graphs, orc, tier, which, off):
+    """Weight sums just below, at and above what the 32-bit form takes (edge
+    sum 2^30, vertex sum 2^28, one weight of 2^31): all equal the oracle."""
+    g = graphs.grid2d(40, 30, weighted=True, seed=8).as_tier(tier)
+    row, adj = g.row.long(), g.adj.long()
+    src = torch.repeat_interleave(torch.arange(g.n), row[1:] - row[:-1])
+
+    def set_edge(u, v, w):
+        g.val[(src == u) & (adj == v)] = w
+        g.val[(src == v) & (adj == u)] = w
+
+    if which == "edges":
+        g.val = g.val * ((1 << 30) // int(g.val.sum()))
+        u, v = 0, int(adj[0])
+        set_edge(u, v, int(g.val[0]) + ((1 << 30) + off - int(g.val.sum())) // 2)
+        assert int(g.val.sum()) == (1 << 30) + off
+    elif which == "vertices":
+        g.vw = g.vw * ((1 << 28) // g.n)
+        g.vw[17] += (1 << 28) + off - int(g.vw.sum())
+        assert int(g.vw.sum()) == (1 << 28) + off
+    else:
+        set_edge(0, int(adj[0]), 1 << 31)
+    og = orc.G.from_csr(g)
+    fn = {"big": jet.partition_big, "biggest": jet.partition_biggest}[tier]
+    for alg in (0, 1):
+        want, wcut, _ = orc.partition(og, 8, alg=alg, imb=1.03, seed=2)
+        part, cut, _ = fn(jet.config_t(coarsening_alg=alg, num_parts=8, max_imb_ratio=1.03), g.to("cuda"), seed=2)
+        assert cut == wcut and np.array_equal(host(part), want)
