@@ -2,6 +2,8 @@
 // Each tier's translation unit instantiates them with its integer types.
 #pragma once
 #include "uncoarsen.cuh"
+#include "stats.cuh"
+#include <algorithm>
 #include <string>
 
 namespace jetb {
@@ -241,59 +243,59 @@ int partition_impl(const jet_config_c* cfg, O n, const E* row, const O* adj, con
 }
 
 // Partition statistics over device arrays (app/part_eval.cpp:73-110,
-// src/part_stat.hpp:77-239).
-template <class O, class E, class W>
-__global__ void k_cut_per_part(GView<O, E, W> g, const part_t* part, W* per) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.n; i += (int64_t)gridDim.x * blockDim.x) {
-        part_t pi = part[i];
-        W acc = 0;
-        for (E j = g.row[i]; j < g.row[i + 1]; j++) if (part[g.adj[j]] != pi) acc += g.val[j];
-        if (acc) atomic_add(&per[pi], acc);
-    }
-}
-template <class O, class E, class W>
-__global__ void k_comm_count(GView<O, E, W> g, const part_t* part, const E* coff, const Slot<W>* slots, const part_t* csize,
-                             long long* out) {
-    long long c = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.n; i += (int64_t)gridDim.x * blockDim.x) {
-        const Slot<W>* b = slots + coff[i];
-        part_t pi = part[i];
-        for (part_t s = 0; s < csize[i]; s++) if (b[s].p >= 0 && b[s].p != pi) c++;
-    }
-    c = group_sum<long long>(c, 32);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd((unsigned long long*)out, (unsigned long long)c);
-}
-
+// src/part_stat.hpp:77-239): the kernels of stats.cuh.
 template <class O, class E, class W>
 void pstat_impl_dev(Engine<O, E, W>& eng, O n, E m, const E* row, const O* adj, const W* val, const W* vw, const part_t* part,
                     part_t k, int64_t* out) {
     cudaStream_t s = eng.s;
+    if (k < 1) throw JetError{JET_ERR_INVALID, "num_parts must be >= 1"};
+    // (the limit of the connectivity tables, which the statistics keep)
+    if (Refiner<O, E, W>::cta_smem_for(k) > (size_t)device_info().max_smem_optin - 1024)
+        throw JetError{JET_ERR_INVALID, "num_parts too large for the shared-memory connectivity tables"};
     Level<O, E, W> L;
     L.n = n; L.m = m; L.row = row; L.adj = adj; L.val = val; L.vw = vw;
     eng.prepare_level(L);
-    Refiner<O, E, W> ref(eng, n, (int64_t)m, k);
-    ref.check_parts(L, part);
-    W cut = ref.total_cut(L, part);
-    DBuf<W> per(k, s);
-    per.zero();
-    k_cut_per_part<O, E, W><<<grid_persistent(n, 8), BLOCK, 0, s>>>(L.view(), part, per.p); count_launch();
+    // cut per part and sizes, then the communication volume and the error flag
+    const int64_t wk = (int64_t)k * 2 * sizeof(W);
+    DBuf<unsigned char> res(wk + 16, s);
+    res.zero();
+    PStatOut<W> po;
+    po.comm = (long long*)res.p;
+    po.bad = (int*)(res.p + 8);
+    po.per = (W*)(res.p + 16);
+    po.sizes = po.per + k;
+    const int hist = wk <= 32 * 1024;
+    const unsigned grid = grid_persistent((int64_t)n * L.group, 8);
+    auto g = L.view();
+    switch (L.group) {
+        case 4: k_pstat_rows<4, O, E, W><<<grid, BLOCK, hist ? wk : 0, s>>>(g, part, k, po, hist); break;
+        case 8: k_pstat_rows<8, O, E, W><<<grid, BLOCK, hist ? wk : 0, s>>>(g, part, k, po, hist); break;
+        case 16: k_pstat_rows<16, O, E, W><<<grid, BLOCK, hist ? wk : 0, s>>>(g, part, k, po, hist); break;
+        default: k_pstat_rows<32, O, E, W><<<grid, BLOCK, hist ? wk : 0, s>>>(g, part, k, po, hist); break;
+    }
+    count_launch();
     JET_LAUNCH_CHECK();
-    std::vector<W> hper(k), hs(k);
-    JET_CUDA(cudaMemcpyAsync(hper.data(), per.p, sizeof(W) * k, cudaMemcpyDeviceToHost, s));
-    ref.part_sizes(L, part, ref.sizes_best.p);
-    JET_CUDA(cudaMemcpyAsync(hs.data(), ref.sizes_best.p, sizeof(W) * k, cudaMemcpyDeviceToHost, s));
-    JET_CUDA(cudaMemcpyAsync(ref.part_work.p, part, sizeof(part_t) * n, cudaMemcpyDeviceToDevice, s));
-    ref.init_conn(L);
-    long long* cc = eng.template dslot<long long>(61);
-    JET_CUDA(cudaMemsetAsync(cc, 0, sizeof(int64_t), s));
-    k_comm_count<O, E, W><<<grid_persistent(n, 8), BLOCK, 0, s>>>(L.view(), part, ref.coff.p, ref.slots.p, ref.csize.p, cc); count_launch();
-    JET_LAUNCH_CHECK();
-    JET_CUDA(cudaMemcpyAsync(&eng.hscal[1], cc, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    const int words = (k + 31) / 32;
+    if (L.n_warp > 0) {
+        k_pstat_long<false, O, E, W><<<grid_persistent((int64_t)L.n_warp * 32, 8), BLOCK, (BLOCK / 32) * words * sizeof(uint32_t), s>>>(
+            g, part, k, L.warp_list.p, L.n_warp, po, words); count_launch();
+        JET_LAUNCH_CHECK();
+    }
+    if (L.n_hub > 0) {
+        k_pstat_long<true, O, E, W><<<(unsigned)std::min<int64_t>((int64_t)L.n_hub, device_info().sms * 2), 1024, words * sizeof(uint32_t), s>>>(
+            g, part, k, L.hub_list.p, L.n_hub, po, words); count_launch();
+        JET_LAUNCH_CHECK();
+    }
+    std::vector<unsigned char> h(wk + 16);
+    JET_CUDA(cudaMemcpyAsync(h.data(), res.p, wk + 16, cudaMemcpyDeviceToHost, s));
     eng.sync();
-    W mx = 0, largest = 0, smallest = std::numeric_limits<W>::max(), total = 0;
-    for (W x : hper) mx = x > mx ? x : mx;
-    for (W x : hs) { largest = x > largest ? x : largest; smallest = x < smallest ? x : smallest; total += x; }
-    out[0] = (int64_t)(cut / 2); out[1] = (int64_t)mx; out[2] = eng.hscal[1];
+    if (*(const int*)(h.data() + 8)) throw JetError{JET_ERR_INVALID, "part id out of range"};
+    const W* per = (const W*)(h.data() + 16);
+    const W* hs = per + k;
+    W cut = 0, mx = 0, largest = 0, smallest = std::numeric_limits<W>::max(), total = 0;
+    for (part_t p = 0; p < k; p++) { cut += per[p]; mx = per[p] > mx ? per[p] : mx; }
+    for (part_t p = 0; p < k; p++) { largest = hs[p] > largest ? hs[p] : largest; smallest = hs[p] < smallest ? hs[p] : smallest; total += hs[p]; }
+    out[0] = (int64_t)(cut / 2); out[1] = (int64_t)mx; out[2] = *(const long long*)h.data();
     out[3] = (int64_t)largest; out[4] = (int64_t)smallest; out[5] = (int64_t)total;
 }
 

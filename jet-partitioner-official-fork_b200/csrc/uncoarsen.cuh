@@ -143,7 +143,8 @@ struct Refiner {
         int kw = k < WARP_TABLE ? k : WARP_TABLE;
         return (size_t)(BLOCK / 32) * kw * (sizeof(part_t) + sizeof(W)) + 16;
     }
-    size_t cta_smem() const { return (((size_t)k * sizeof(part_t) + 15) & ~(size_t)15) + (size_t)k * sizeof(W); }
+    static size_t cta_smem_for(part_t k) { return (((size_t)k * sizeof(part_t) + 15) & ~(size_t)15) + (size_t)k * sizeof(W); }
+    size_t cta_smem() const { return cta_smem_for(k); }
 
     bool attrs_done = false;
     void set_attrs() {

@@ -687,3 +687,21 @@ def test_32_bit_rule_at_its_edges(jet, graphs, orc, tier, which, off):
         want, wcut, _ = orc.partition(og, 8, alg=alg, imb=1.03, seed=2)
         part, cut, _ = fn(jet.config_t(coarsening_alg=alg, num_parts=8, max_imb_ratio=1.03), g.to("cuda"), seed=2)
         assert cut == wcut and np.array_equal(host(part), want)
+
+
+@pytest.mark.parametrize("tier", TIERS)
+@pytest.mark.parametrize("kind", ["grid2d", "grid3d", "rgg", "rmat", "star", "dense"])
+@pytest.mark.parametrize("k", [2, 31, 33, 700, 5000])
+def test_pstat_row_classes(jet, graphs, orc, tier, kind, k):
+    """Statistics of rows in every class (register compare, warp and block
+    bitmaps; histograms in shared and in global memory), of slabs and of
+    scattered parts; a part id out of range is refused."""
+    g = make(graphs, kind, tier)
+    og = orc.G.from_csr(g)
+    rng = np.random.default_rng(k)
+    slabs = (np.arange(g.n) * min(k, g.n) // g.n).astype(np.int32)
+    for part in (rng.integers(0, k, g.n).astype(np.int32), slabs):
+        assert jet.pstat(g.to("cuda"), torch.from_numpy(part).cuda(), k) == orc.pstat(og, part, k).tolist()
+    part[g.n // 2] = k
+    with pytest.raises(jet.JetError):
+        jet.pstat(g.to("cuda"), torch.from_numpy(part).cuda(), k)
