@@ -213,7 +213,9 @@ __device__ __forceinline__ bool coop_reb_tail(RefArgs<O, E, W>& a, RebArgs<O, W>
         // (classification, ordering, eviction, cookie cutter, destinations)
         // read the copy of their own block
         W* boff_s = (W*)(smem_raw + cs.boff_off);
-        block_scan_global<W>(rb.buckets, boff_s, (int64_t)rb.t_minibuckets + 1);
+        const int64_t nb = (int64_t)rb.t_minibuckets + 1;
+        if (nb > 4 * (int64_t)blockDim.x) block_scan_long<W>(rb.buckets, boff_s, nb);
+        else block_scan_global<W>(rb.buckets, boff_s, nb);
         rb.boff = boff_s;
     } else if (!grid_scan<CL, W>(GetArray<W>{rb.buckets}, (int64_t)rb.t_minibuckets + 1, rb.boff, cs.wsum, cs.bar, err)) {
         return false;

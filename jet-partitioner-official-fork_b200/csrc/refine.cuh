@@ -115,6 +115,7 @@ struct RefArgs {
     RefDev<O, W>* dev;
     const double* filter;  // LP filter ratio, read on the device (it changes per iteration with ultra settings)
     int narrow;            // every row's summed edge weight fits in 32 bits (see acc_add)
+    part_t tw;             // entries of a warp's shared-memory table (warp_table_width)
     unsigned long long* pclk;  // per-phase clock totals of the persistent level loops, or null (jet_prof_phases)
 };
 
@@ -361,8 +362,18 @@ __device__ __forceinline__ int table_add_edges(const RefArgs<O, E, W>& a, part_t
     return mine;
 }
 
-// 32 < deg <= 4096 and k <= WARP_TABLE: one warp per vertex, table in shared memory.
+// 32 < deg <= 4096 and warp_table_width <= WARP_TABLE: one warp per vertex,
+// table in shared memory.
 static constexpr int WARP_TABLE = 512;
+// Entries each warp of conn_warp_row needs on a level: its rows with 4 * cap <
+// k take a hash table and its rehash (2 * cap), any other row k. On meshes
+// the rows stay short, so even k of many hundreds needs few entries.
+template <class E>
+__host__ __device__ __forceinline__ part_t warp_table_width(E max_deg, part_t k) {
+    const part_t cap = conn_cap<E>(max_deg, k);
+    if (4 * (int64_t)cap >= (int64_t)k) return k;
+    return cap > 0 ? 2 * cap : 1;
+}
 
 // Writes a row's table from a direct-mapped accumulator: vals[p] is the
 // row's summed weight to part p (p < k; zero = absent).  A table of size k
@@ -456,7 +467,7 @@ __device__ __forceinline__ void hashed_table_write(part_t* keys, W* vals, part_t
 }
 
 // One row's table built by one warp in its own shared-memory slice (`keys`,
-// `vals`: k entries each, k <= WARP_TABLE; vals all zero on entry, and left
+// `vals`: warp_table_width entries each; vals all zero on entry, and left
 // all zero).  Rows with cap >= k / 4: every edge adds its weight at its
 // part's index (no hashing, no slot claiming), the nonzero entries are
 // counted, and the table is written by direct_table_write, which clears what
@@ -510,7 +521,7 @@ __device__ __forceinline__ void d_conn_warp(RefArgs<O, E, W> a, const O* list, O
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (gate && !*gate) return;
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kw = a.k < WARP_TABLE ? a.k : WARP_TABLE;
+    const int kw = a.tw;
     const int nw = (int)(blockDim.x >> 5);
     part_t* keys = (part_t*)smem_raw + wid * kw;
     W* vals = (W*)(smem_raw + (((size_t)nw * kw * sizeof(part_t) + 15) & ~(size_t)15)) + wid * kw;
@@ -1392,12 +1403,28 @@ __device__ __forceinline__ int chunk_scan(const W* es, int p, int k, W sc) {
     return lo - 1;
 }
 
+// chunk_scan for a replay, whose positions never decrease: `q` is the last
+// index with es[q] <= sc so far and `next` = es[q + 1]. As long as es[p] <= sc
+// (every first position lies before the cursor) the scan's result is that
+// index whatever p is, so it is found by walking q on instead of a binary
+// search per draw, each step of which waited for the last one's load.
+template <class W>
+__device__ __forceinline__ int chunk_walk(const W* es, int p, int k, W sc, int& q, W& next) {
+    if (p > k || es[p] > sc) return p - 1;
+    while (q < k && next <= sc) {
+        q++;
+        next = q < k ? es[q + 1] : W(0);
+    }
+    return q;
+}
+
 // The replay is one thread's serial walk (each draw advances the shared
 // cursor), so what it reads is staged first: the chunk bounds in shared
 // memory (when k fits) and, given `stage` shared memory for it, each queued
 // vertex's weight and chunk, with the chosen chunks written back there and
 // stored by the whole block; without it each vertex's data is loaded one
-// vertex ahead of its use.
+// vertex ahead of its use.  717k-vertex mesh into 768 parts: 44.6 us per
+// replay with a binary search in global memory for every draw, 25.9 us now.
 static constexpr int REDRAW_ES_CAP = 513;
 template <class O, class E, class W>
 __device__ __forceinline__ void d_strong_redraw(RefArgs<O, E, W> a, RebArgs<O, W> rb, unsigned char* stage = nullptr,
@@ -1406,10 +1433,15 @@ __device__ __forceinline__ void d_strong_redraw(RefArgs<O, E, W> a, RebArgs<O, W
     __shared__ W es_s[REDRAW_ES_CAP];
     O cnt = a.dev->nredraw;
     if (cnt == 0) return;
+    // the chunk bounds: in the fixed buffer, else at the front of the stage
+    const size_t es_bytes = ((size_t)(a.k + 1) * sizeof(W) + 15) & ~(size_t)15;
     const bool es_in = a.k + 1 <= REDRAW_ES_CAP;
-    if (es_in)
-        for (int p = threadIdx.x; p <= a.k; p += blockDim.x) es_s[p] = rb.evict_start[p];
-    const W* es = es_in ? es_s : rb.evict_start;
+    const bool es_stage = !es_in && stage && es_bytes <= stage_bytes;
+    W* es_dst = es_in ? es_s : (W*)stage;
+    if (es_in || es_stage)
+        for (int p = threadIdx.x; p <= a.k; p += blockDim.x) es_dst[p] = rb.evict_start[p];
+    const W* es = es_in || es_stage ? es_dst : rb.evict_start;
+    if (es_stage) { stage += es_bytes; stage_bytes -= es_bytes; }
     bool fits = cnt <= REDRAW_CAP;
     if (fits) {
         int P = 1;
@@ -1432,6 +1464,8 @@ __device__ __forceinline__ void d_strong_redraw(RefArgs<O, E, W> a, RebArgs<O, W
         __syncthreads();
         if (threadIdx.x == 0) {
             W cursor = a.dev->vw_cursor;
+            int q = chunk_scan<W>(es, 0, a.k, cursor);
+            W next = q < a.k ? es[q + 1] : W(0);
             for (int x = 0; x < (int)cnt; x++) {
                 const W w = sw[x];
                 int p = sp[x];
@@ -1440,8 +1474,8 @@ __device__ __forceinline__ void d_strong_redraw(RefArgs<O, E, W> a, RebArgs<O, W
                 while (p < a.k) {
                     W sc = cursor;
                     cursor += w;
-                    p = chunk_scan<W>(es, p, a.k, sc);
-                    if (p < a.k && w / 2 <= es[p + 1] - sc) { dest = p; break; }
+                    p = chunk_walk<W>(es, p, a.k, sc, q, next);
+                    if (p < a.k && w / 2 <= (p == q ? next : es[p + 1]) - sc) { dest = p; break; }
                     if (++guard > 4 * a.k + 64) { atomicOr(&a.dev->err, ERRF_SPIN); break; }
                 }
                 sp[x] = dest;
@@ -1457,6 +1491,8 @@ __device__ __forceinline__ void d_strong_redraw(RefArgs<O, E, W> a, RebArgs<O, W
     }
     if (threadIdx.x != 0) return;
     W cursor = a.dev->vw_cursor;
+    int q = chunk_scan<W>(es, 0, a.k, cursor);
+    W next = q < a.k ? es[q + 1] : W(0);
     O v = fits ? list[0] : rb.redraw[0];
     W w = a.g.vw[v];
     int p = rb.redraw_p[v];
@@ -1477,7 +1513,7 @@ __device__ __forceinline__ void d_strong_redraw(RefArgs<O, E, W> a, RebArgs<O, W
         while (p < a.k) {
             W sc = cursor;
             cursor += w;
-            p = chunk_scan<W>(es, p, a.k, sc);
+            p = chunk_walk<W>(es, p, a.k, sc, q, next);
             if (p < a.k && w / 2 <= es[p + 1] - sc) { dest = p; break; }
             if (++guard > 4 * a.k + 64) { atomicOr(&a.dev->err, ERRF_SPIN); break; }
         }

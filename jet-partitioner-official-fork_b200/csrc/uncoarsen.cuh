@@ -135,13 +135,14 @@ struct Refiner {
         a.pregain = pregain.p; a.sizes = sizes_curr.p; a.cand = cand.p; a.cand_hub = cand_hub.p; a.moves = moves.p;
         a.moves_hub = moves_hub.p; a.dev = dev.p; a.filter = &ctl.p->filter;
         a.narrow = narrow_state > 0 ? 1 : 0;
+        a.tw = table_width(L);
         a.pclk = phase_clk_ptr();
         return a;
     }
 
-    size_t warp_smem() const {
-        int kw = k < WARP_TABLE ? k : WARP_TABLE;
-        return (size_t)(BLOCK / 32) * kw * (sizeof(part_t) + sizeof(W)) + 16;
+    part_t table_width(const Level<O, E, W>& L) const { return warp_table_width<E>(L.max_deg, k); }
+    size_t warp_smem(const Level<O, E, W>& L) const {
+        return (size_t)(BLOCK / 32) * table_width(L) * (sizeof(part_t) + sizeof(W)) + 16;
     }
     static size_t cta_smem_for(part_t k) { return (((size_t)k * sizeof(part_t) + 15) & ~(size_t)15) + (size_t)k * sizeof(W); }
     size_t cta_smem() const { return cta_smem_for(k); }
@@ -183,8 +184,8 @@ struct Refiner {
             return;
         }
         if (L.n_warp > 0) {
-            if (k <= WARP_TABLE) {
-                k_conn_warp<O, E, W><<<grid_persistent((int64_t)L.n_warp * 32, 16), BLOCK, warp_smem(), s>>>(a, L.warp_list.p, L.n_warp, only_marked, gate, INT64_MAX); count_launch();
+            if (a.tw <= WARP_TABLE) {
+                k_conn_warp<O, E, W><<<grid_persistent((int64_t)L.n_warp * 32, 16), BLOCK, warp_smem(L), s>>>(a, L.warp_list.p, L.n_warp, only_marked, gate, INT64_MAX); count_launch();
             } else {
                 k_conn_cta<O, E, W><<<grid_for(L.n_warp, 1) < 4096 ? grid_for(L.n_warp, 1) : 4096, 256, cta_smem(), s>>>(a, L.warp_list.p, L.n_warp, only_marked, gate, 0, 0); count_launch();
             }
@@ -196,7 +197,7 @@ struct Refiner {
             // only the longest rows get a whole CTA
             int64_t cta_from = 0;
             if (k <= WARP_TABLE) {
-                k_conn_warp<O, E, W><<<grid_persistent((int64_t)L.n_hub * 32, 16), BLOCK, warp_smem(), s>>>(a, L.hub_list.p, L.n_hub, only_marked, gate, WARP_ROW_MAX); count_launch();
+                k_conn_warp<O, E, W><<<grid_persistent((int64_t)L.n_hub * 32, 16), BLOCK, warp_smem(L), s>>>(a, L.hub_list.p, L.n_hub, only_marked, gate, WARP_ROW_MAX); count_launch();
                 cta_from = WARP_ROW_MAX;
             }
             if ((int64_t)L.max_deg > cta_from) {
@@ -781,7 +782,7 @@ struct Refiner {
     static int64_t cluster_max_m() { static const int64_t v = bound("JET_PERSISTENT_MAX_M", CLUSTER_MAX_M); return v; }
     static int64_t coop_max_m() { static const int64_t v = bound("JET_PERSISTENT_MAX_M", COOP_MAX_M); return v; }
     bool cta_eligible(const Level<O, E, W>& L) const {
-        int64_t cap = (use_cluster && !batch_thread() && cluster_size() > 0) ? cta_prefer_n() : CTA_MAX_N;
+        int64_t cap = (use_cluster && !batch_thread() && cluster_size(L) > 0) ? cta_prefer_n() : CTA_MAX_N;
         return use_cta && (int64_t)L.n <= cap && (int64_t)L.m <= CTA_MAX_M && k <= CTA_MAX_K;
     }
 
@@ -817,7 +818,7 @@ struct Refiner {
         RebArgs<O, W> rbs = reb_args(L, strong_max_dest(pb.opt, pb.size_max), pb.opt, pb.size_max, false);
         int P = 1;
         while (P < (int)L.n) P <<= 1;
-        size_t scratch = level_cta_smem<O, W>(P, k) + 64;
+        size_t scratch = level_cta_smem<O, W>(P, table_width(L)) + 64;
         // the attribute is per function and process-wide: always the device
         // maximum, so concurrent callers with different sizes cannot race
         const size_t smax = max_dynamic_smem((const void*)k_level_cta<O, E, W>);
@@ -838,9 +839,16 @@ struct Refiner {
     // vertex level, 3.1 M entries, runs 86 against 111 us per iteration here;
     // the 749,582-vertex level gains nothing and the 2 M one loses).
     static constexpr int64_t COOP_MAX_N = (int64_t)1 << 18;
+    // Parts up to which the persistent loops take a level whose rows fit the
+    // warps' shared-memory tables. 717k-vertex mesh into 768 parts: its levels
+    // of 1,323-61,159 vertices ran 98-297 us per iteration as level graphs
+    // and run 89-171 on the cluster (the whole call 161.6 -> 151.0 ms, of
+    // which Metis 73); beyond about 1,000 parts the bucket arrays (50 per part
+    // and section) outgrow the blocks' shared memory and the gain.
+    static constexpr part_t LEVEL_MAX_K = 1024;
     static constexpr int64_t COOP_MAX_M = (int64_t)1 << 22;
-    size_t coop_smem() const {
-        int kw = k < WARP_TABLE ? k : WARP_TABLE;
+    size_t coop_smem(const Level<O, E, W>& L) const {
+        size_t kw = (size_t)table_width(L);
         size_t nw = CTA_THREADS / 32;
         size_t conn = ((nw * kw * sizeof(part_t) + 15) & ~(size_t)15) + nw * kw * sizeof(W);
         size_t q = (size_t)coop_boff_off() + (size_t)coop_boff_cap() * sizeof(W);
@@ -861,7 +869,7 @@ struct Refiner {
     int coop_qcap() const { return COOP_QUEUE_KEYS; }
     // bucket offsets every block of the persistent grid keeps in shared
     // memory after the keys: room for the largest level the grid drivers
-    // take, within 128 KiB (else those levels scan them across the grid)
+    // take, within 160 KiB (else those levels scan them across the grid)
     int64_t coop_boff_cap() const {
         int64_t nmax = (int64_t)n_max;
         const int64_t lim = coop_max_n() > cluster_max_n() ? coop_max_n() : cluster_max_n();
@@ -869,7 +877,7 @@ struct Refiner {
         O sections, tmb;
         sections_for((O)nmax, sections, tmb);
         const int64_t want = (int64_t)tmb + 1;
-        return want * (int64_t)sizeof(W) <= ((int64_t)128 << 10) ? want : 0;
+        return want * (int64_t)sizeof(W) <= ((int64_t)160 << 10) ? want : 0;
     }
     size_t coop_static_smem() const {
         static size_t bytes = [] {
@@ -880,8 +888,8 @@ struct Refiner {
     }
     bool coop_eligible(const Level<O, E, W>& L) const {
         return use_coop && device_info().coop && !cta_eligible(L) && (int64_t)L.n <= coop_max_n() &&
-               (int64_t)L.m <= coop_max_m() && k <= WARP_TABLE &&
-               coop_smem() + coop_static_smem() <= (size_t)device_info().max_smem_optin;
+               (int64_t)L.m <= coop_max_m() && k <= LEVEL_MAX_K && table_width(L) <= WARP_TABLE &&
+               coop_smem(L) + coop_static_smem() <= (size_t)device_info().max_smem_optin;
     }
 
     // ------------------------------------------------------------ cluster loop
@@ -893,9 +901,12 @@ struct Refiner {
     // CTAs in the level cluster: 16 where the device allows it, else 8, 0 if
     // no cluster of 1024-thread CTAs with this shared memory fits.
     mutable int cluster_cache = -1;
-    int cluster_size() const {
-        if (cluster_cache >= 0) return cluster_cache;
-        cluster_cache = [this] {
+    mutable size_t cluster_cache_smem = 0;
+    int cluster_size(const Level<O, E, W>& L) const {
+        const size_t smem = coop_smem(L);
+        if (cluster_cache >= 0 && cluster_cache_smem == smem) return cluster_cache;
+        cluster_cache_smem = smem;
+        cluster_cache = [smem] {
             const void* f = (const void*)k_level_coop<true, O, E, W>;
             if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem(f)) != cudaSuccess) return 0;
             cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -903,7 +914,7 @@ struct Refiner {
                 cudaLaunchConfig_t cfg = {};
                 cfg.gridDim = dim3(want);
                 cfg.blockDim = dim3(CTA_THREADS);
-                cfg.dynamicSmemBytes = coop_smem();
+                cfg.dynamicSmemBytes = smem;
                 cudaLaunchAttribute at;
                 at.id = cudaLaunchAttributeClusterDimension;
                 at.val.clusterDim.x = want;
@@ -921,8 +932,8 @@ struct Refiner {
     }
     bool cluster_eligible(const Level<O, E, W>& L) const {
         return use_cluster && !cta_eligible(L) && (int64_t)L.n <= cluster_max_n() && (int64_t)L.m <= cluster_max_m() &&
-               k <= WARP_TABLE &&
-               coop_smem() + coop_static_smem() <= (size_t)device_info().max_smem_optin && cluster_size() > 0;
+               k <= LEVEL_MAX_K && table_width(L) <= WARP_TABLE &&
+               coop_smem(L) + coop_static_smem() <= (size_t)device_info().max_smem_optin && cluster_size(L) > 0;
     }
 
     // The whole level loop as one persistent launch: a single cluster
@@ -930,10 +941,10 @@ struct Refiner {
     // (bounded software barriers).
     void run_level_coop(const Level<O, E, W>& L, part_t* best_part, const Prob& pb, const std::vector<double>& temps, double tol,
                         bool cluster = false) {
-        size_t smem = coop_smem();
+        size_t smem = coop_smem(L);
         int grid = 0;
         if (cluster) {
-            grid = cluster_size();
+            grid = cluster_size(L);
         } else {
             JET_CUDA(cudaFuncSetAttribute(k_level_coop<false, O, E, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           max_dynamic_smem((const void*)k_level_coop<false, O, E, W>)));

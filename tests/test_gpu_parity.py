@@ -705,3 +705,60 @@ def test_pstat_row_classes(jet, graphs, orc, tier, kind, k):
     part[g.n // 2] = k
     with pytest.raises(jet.JetError):
         jet.pstat(g.to("cuda"), torch.from_numpy(part).cuda(), k)
+
+
+def _partition_with(jet, mask, tier, cfg, g, seed):
+    prev = jet.set_refine_drivers(mask)
+    try:
+        fn = {"i32": jet.partition, "big": jet.partition_big, "biggest": jet.partition_biggest}[tier]
+        part, cut, _ = fn(cfg, g.to("cuda"), seed=seed)
+    finally:
+        jet.set_refine_drivers(prev)
+    return host(part), cut
+
+
+@pytest.mark.parametrize("drivers", ["all", "cluster", "coop", "host"])
+@pytest.mark.parametrize("tier,kind,k", [("i32", "grid3d", 513), ("i32", "rgg", 1024), ("i32", "rgg", 1025), ("big", "rgg", 700),
+                                         ("i32", "hubs", 600)])
+def test_many_parts_on_the_persistent_loops(jet, graphs, orc, drivers, tier, kind, k):
+    """k above a warp table's 512 entries: levels of short rows run on the
+    persistent loops with hash tables of twice the largest row ("hubs": a
+    graph with longer rows, which needs k entries and keeps the other
+    drivers); all equal the oracle."""
+    q = jet.DRIVER_REB_QUEUE
+    mask = {"all": jet.DRIVER_ALL, "cluster": jet.DRIVER_CLUSTER | q, "coop": jet.DRIVER_COOP | jet.DRIVER_GRAPH | q,
+            "host": q}[drivers]
+    if kind == "grid3d":
+        g = graphs.grid3d(30, 30, 31, weighted=True, seed=2)
+    elif kind == "rgg":
+        g = graphs.rgg(30000, 9.0, seed=5)
+    else:
+        gen = torch.Generator().manual_seed(4)
+        n = 20000
+        u = torch.cat([torch.arange(n), torch.arange(20).repeat_interleave(300)])
+        v = torch.cat([(torch.arange(n) + 1) % n, torch.randint(0, n, (6000,), generator=gen)])
+        a, b = torch.minimum(u, v), torch.maximum(u, v)
+        pairs = torch.unique((a * n + b)[a != b])
+        g = graphs.from_undirected(n, pairs // n, pairs % n, torch.randint(1, 9, (pairs.numel(),), generator=gen))
+    g = g.as_tier(tier)
+    cfg = jet.config_t(coarsening_alg=1, num_parts=k, max_imb_ratio=1.05)
+    want, wcut, _ = orc.partition(orc.G.from_csr(g), k, alg=1, imb=1.05, seed=4)
+    part, cut = _partition_with(jet, mask, tier, cfg, g, 4)
+    assert cut == wcut and np.array_equal(part, want)
+
+
+@pytest.mark.parametrize("drivers", ["all", "cta_global", "cluster", "coop", "graph", "host_fullsort"])
+@pytest.mark.parametrize("tier,k", [("big", 64), ("biggest", 600)])
+def test_level_drivers_64_bit(jet, graphs, orc, drivers, tier, k):
+    """The 64-bit instantiations of the level drivers: edge weights whose sum
+    does not fit 32 bits."""
+    q = jet.DRIVER_REB_QUEUE
+    mask = {"all": jet.DRIVER_ALL, "cta_global": jet.DRIVER_CTA | q, "cluster": jet.DRIVER_CLUSTER | q,
+            "coop": jet.DRIVER_COOP | jet.DRIVER_GRAPH | q, "graph": jet.DRIVER_GRAPH | q, "host_fullsort": 0}[drivers]
+    g = graphs.rgg(20000, 9.0, seed=5).as_tier(tier)
+    g.val = g.val * 100003
+    assert int(g.val.sum()) > 1 << 31
+    cfg = jet.config_t(coarsening_alg=0, num_parts=k, max_imb_ratio=1.03)
+    want, wcut, _ = orc.partition(orc.G.from_csr(g), k, alg=0, imb=1.03, seed=3)
+    part, cut = _partition_with(jet, mask, tier, cfg, g, 3)
+    assert cut == wcut and np.array_equal(part, want)
