@@ -116,6 +116,7 @@ struct RefArgs {
     const double* filter;  // LP filter ratio, read on the device (it changes per iteration with ultra settings)
     int narrow;            // every row's summed edge weight fits in 32 bits (see acc_add)
     part_t tw;             // entries of a warp's shared-memory table (warp_table_width)
+    int mixed;             // the level has rows of degree > THREAD_DEG (left to the warp kernels)
     unsigned long long* pclk;  // per-phase clock totals of the persistent level loops, or null (jet_prof_phases)
 };
 
@@ -770,21 +771,22 @@ __device__ __forceinline__ bool lp_better(W c, part_t e, W bc, part_t be) {
     return c > 0 && (c > bc || (c == bc && e < be));
 }
 
+// Filters a computed destination (`best` becomes NO_MOVE when it fails) and
+// caches it with its gain, which is returned.  Only candidates' entries of
+// a.dest are read (afterburner, moves), so the callers write those alone.
 template <class O, class E, class W>
-__device__ __forceinline__ void lp_finish(const RefArgs<O, E, W>& a, O i, part_t best, W b_conn, W p_conn, double filter_ratio,
-                                          bool computed) {
-    if (computed) {
-        W sg = 0;
-        if (best != NO_MOVE) {
-            if (b_conn >= p_conn || ((double)(p_conn - b_conn) < floor(filter_ratio * (double)p_conn))) sg = b_conn - p_conn;
-            else best = NO_MOVE;
-        }
-        a.save_gain[i] = sg;
-        a.dest_cache[i] = best;
+__device__ __forceinline__ W lp_finish(const RefArgs<O, E, W>& a, O i, part_t& best, W b_conn, W p_conn, double filter_ratio) {
+    W sg = 0;
+    if (best != NO_MOVE) {
+        if (b_conn >= p_conn || ((double)(p_conn - b_conn) < floor(filter_ratio * (double)p_conn))) sg = b_conn - p_conn;
+        else best = NO_MOVE;
     }
-    a.dest[i] = best;
+    a.save_gain[i] = sg;
+    a.dest_cache[i] = best;
+    return sg;
 }
 
+// One vertex per thread and round (the persistent level loops).
 template <class O, class E, class W>
 __device__ __forceinline__ void d_lp_select_thread(RefArgs<O, E, W> a) {
     const W GAIN_MIN = std::numeric_limits<W>::lowest();
@@ -798,8 +800,10 @@ __device__ __forceinline__ void d_lp_select_thread(RefArgs<O, E, W> a) {
         O i = (O)x;
         if (x < a.g.n && a.g.row[i + 1] - a.g.row[i] <= THREAD_DEG) {
             part_t best = a.dest_cache[i];
+            const uint8_t lk = a.lock[i];
+            W gain = 0;
             if (best != NULL_PART) {
-                lp_finish<O, E, W>(a, i, best, 0, 0, filter_ratio, false);
+                if (best >= 0 && lk == 0) gain = a.save_gain[i];
             } else {
                 part_t p = a.part[i];
                 best = NO_MOVE;
@@ -810,19 +814,181 @@ __device__ __forceinline__ void d_lp_select_thread(RefArgs<O, E, W> a) {
                     if (sl.p != p) { if (lp_better<W>(sl.v, sl.p, b_conn, best)) { best = sl.p; b_conn = sl.v; } }
                     else if (sl.v > 0) p_conn = sl.v;
                 });
-                lp_finish<O, E, W>(a, i, best, b_conn, p_conn, filter_ratio, true);
-                best = a.dest[i];
+                gain = lp_finish<O, E, W>(a, i, best, b_conn, p_conn, filter_ratio);
             }
-            cand = best != NO_MOVE && a.lock[i] == 0;
-            if (cand) a.pregain[i] = a.save_gain[i];
-            else { a.pregain[i] = GAIN_MIN; a.lock[i] = 0; }
+            cand = best != NO_MOVE && lk == 0;
+            a.pregain[i] = cand ? gain : GAIN_MIN;
+            if (cand) a.dest[i] = best;
+            else if (lk) a.lock[i] = 0;
         }
         O s = warp_append(&a.dev->ncand, cand);
         if (cand) a.cand[s] = i;
     }
 }
+// ---- passes over every vertex of a level
+// Most vertices need a few bytes (a cached destination, a part below its
+// bound) and some their whole table. With one vertex per thread and round the
+// passes were chains of dependent loads, and a warp waited for its slowest
+// row. Here a warp owns a stretch of consecutive vertices, loads PASS_U of
+// them per lane before the first use, finishes the light ones and collects
+// the others in shared memory; those are then dealt to the lanes, several to
+// a vertex where few are left (PassDeal).
+// These are the grid kernels' forms: on the 2.1 M-vertex level of the 128^3
+// mesh an iteration went from 128 to 118 us, on R-MAT 2^24's finest level from
+// 5.69 to 5.47 ms. The persistent level loops keep one vertex per thread: their
+// levels have one to two rounds, nothing to overlap, and the longer code cost
+// them 2-3 us a pass (one CTA: LP select 2.8 -> 6.1 us, classification 1.1 -> 3.0).
+// `list`: 32 * PASS_U bytes of shared memory per warp.
+static constexpr int PASS_U = 4;
+static constexpr int PASS_LIST = 32 * PASS_U;
+struct WarpPass {
+    int64_t n, warps, w;
+    int64_t rounds;
+    int chunk;  // vertices per warp and round, at most 32 * PASS_U
+    __device__ __forceinline__ WarpPass(int64_t count, int64_t start, int64_t stride) : n(count), warps(stride >> 5), w(start >> 5) {
+        constexpr int FULL = 32 * PASS_U;
+        if (n <= warps * FULL) {
+            rounds = 1;
+            chunk = (int)((unsigned)(n + warps - 1) / (unsigned)warps);
+        } else {
+            rounds = ceil_div<int64_t>(n, warps * FULL);
+            chunk = (int)ceil_div<int64_t>(n, warps * rounds);
+        }
+        if (chunk > 32) chunk = (chunk + 31) & ~31;
+    }
+    __device__ __forceinline__ int64_t base(int64_t r) const { return (r * warps + w) * chunk; }
+    __device__ __forceinline__ int count(int64_t base) const {
+        const int64_t left = n - base;
+        return left <= 0 ? 0 : (left < chunk ? (int)left : chunk);
+    }
+};
+// Lanes per collected vertex: the largest power of two that deals all of
+// them at once, else one.
+struct PassDeal {
+    int g, per, slot, sub;
+    __device__ __forceinline__ PassDeal(int cnt, int lane) {
+        g = 32;
+        while (g > 1 && cnt * g > 32) g >>= 1;
+        per = 32 / g;
+        sub = lane & (g - 1);
+        slot = lane / g;
+    }
+};
+// Visits slots sub, sub + g, ... < sz of a table, four loads ahead of use.
+template <class W, class F>
+__device__ __forceinline__ void scan_slots_part(const Slot<W>* base, part_t sz, int sub, int g, F&& body) {
+    for (part_t s0 = sub; s0 < sz; s0 += 4 * g) {
+        Slot<W> sl[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (s0 + u * g < sz) sl[u] = base[s0 + u * g];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (s0 + u * g < sz) body(sl[u]);
+    }
+}
+
 template <class O, class E, class W>
-__global__ void __launch_bounds__(BLOCK) k_lp_select_thread(RefArgs<O, E, W> a) { d_lp_select_thread<O, E, W>(a); }
+__device__ __forceinline__ void d_lp_select_pass(RefArgs<O, E, W> a, uint8_t* list) {
+    const W GAIN_MIN = std::numeric_limits<W>::lowest();
+    const double filter_ratio = *a.filter;
+    const int lane = threadIdx.x & 31;
+    const unsigned before = (1u << lane) - 1;
+    uint8_t* sel = list + (threadIdx.x >> 5) * PASS_LIST;
+    const WarpPass wp((int64_t)a.g.n, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+    for (int64_t r = 0; r < wp.rounds; r++) {
+        const int64_t b0 = wp.base(r);
+        const int cnt = wp.count(b0);
+        if (cnt == 0) break;
+        part_t best[PASS_U];
+        uint8_t lk[PASS_U];
+        bool in[PASS_U];
+        W sg[PASS_U];
+#pragma unroll
+        for (int u = 0; u < PASS_U; u++) {
+            const int64_t i = b0 + u * 32 + lane;
+            in[u] = u * 32 + lane < cnt;
+            best[u] = in[u] ? a.dest_cache[i] : NO_MOVE;
+            lk[u] = in[u] ? a.lock[i] : (uint8_t)0;
+            if (a.mixed && in[u]) in[u] = a.g.row[i + 1] - a.g.row[i] <= THREAD_DEG;
+        }
+#pragma unroll
+        for (int u = 0; u < PASS_U; u++)
+            sg[u] = in[u] && best[u] >= 0 && !lk[u] ? a.save_gain[b0 + u * 32 + lane] : (W)0;
+        int nh = 0, nc = 0, at[PASS_U];
+#pragma unroll
+        for (int u = 0; u < PASS_U; u++) {
+            const int64_t i = b0 + u * 32 + lane;
+            const bool heavy = in[u] && best[u] == NULL_PART;
+            const bool cand = in[u] && best[u] >= 0 && !lk[u];
+            const unsigned hm = __ballot_sync(0xffffffffu, heavy), cm = __ballot_sync(0xffffffffu, cand);
+            if (heavy) sel[nh + __popc(hm & before)] = (uint8_t)(u * 32 + lane);
+            at[u] = cand ? nc + __popc(cm & before) : -1;
+            if (cand) {
+                a.dest[i] = best[u];
+                a.pregain[i] = sg[u];
+            } else if (in[u] && !heavy) {
+                a.pregain[i] = GAIN_MIN;
+                if (lk[u]) a.lock[i] = 0;
+            }
+            nh += __popc(hm);
+            nc += __popc(cm);
+        }
+        if (nc) {
+            O first = 0;
+            if (lane == 0) first = atomic_add(&a.dev->ncand, (O)nc);
+            first = __shfl_sync(0xffffffffu, first, 0);
+#pragma unroll
+            for (int u = 0; u < PASS_U; u++)
+                if (at[u] >= 0) a.cand[first + at[u]] = (O)(b0 + u * 32 + lane);
+        }
+        __syncwarp();
+        const PassDeal d(nh, lane);
+        for (int x0 = 0; x0 < nh; x0 += d.per) {
+            const bool act = x0 + d.slot < nh;
+            O i = 0;
+            part_t p = 0, sz = 0, bp = NO_MOVE;
+            const Slot<W>* base = nullptr;
+            uint8_t l = 0;
+            if (act) {
+                i = (O)(b0 + sel[x0 + d.slot]);
+                p = a.part[i];
+                base = a.slots + a.coff[i];
+                sz = a.csize[i];
+                l = a.lock[i];
+            }
+            W b_conn = 0, p_conn = 0;
+            scan_slots_part<W>(base, sz, d.sub, d.g, [&](const Slot<W>& sl) {
+                if (sl.p != p) { if (lp_better<W>(sl.v, sl.p, b_conn, bp)) { bp = sl.p; b_conn = sl.v; } }
+                else if (sl.v > 0) p_conn = sl.v;
+            });
+            for (int m = d.g >> 1; m > 0; m >>= 1) {
+                const W c2 = shfl_xor(b_conn, m, 32);
+                const part_t e2 = shfl_xor(bp, m, 32);
+                if (lp_better<W>(c2, e2, b_conn, bp)) { b_conn = c2; bp = e2; }
+                const W pc2 = shfl_xor(p_conn, m, 32);
+                if (pc2 > p_conn) p_conn = pc2;
+            }
+            const bool own = act && d.sub == 0;
+            bool cand = false;
+            if (own) {
+                const W gain = lp_finish<O, E, W>(a, i, bp, b_conn, p_conn, filter_ratio);
+                cand = bp != NO_MOVE && l == 0;
+                a.pregain[i] = cand ? gain : GAIN_MIN;
+                if (cand) a.dest[i] = bp;
+                else if (l) a.lock[i] = 0;
+            }
+            const O s = warp_append(&a.dev->ncand, cand);
+            if (cand) a.cand[s] = i;
+        }
+        __syncwarp();
+    }
+}
+template <class O, class E, class W>
+__global__ void __launch_bounds__(BLOCK) k_lp_select_thread(RefArgs<O, E, W> a) {
+    __shared__ uint8_t list[BLOCK / 32 * PASS_LIST];
+    d_lp_select_pass<O, E, W>(a, list);
+}
 
 // Vertices with deg > 32: one warp per vertex scans its table.
 template <class O, class E, class W>
@@ -834,19 +1000,18 @@ __device__ __forceinline__ void d_lp_select_warp(RefArgs<O, E, W> a, const O* li
     for (int64_t x = blockIdx.x * (int64_t)(int)(blockDim.x >> 5) + (threadIdx.x >> 5); x < count; x += warps) {
         O i = list[x];
         part_t best = a.dest_cache[i];
+        const uint8_t lk = a.lock[i];
+        W gain = 0;
         if (best != NULL_PART) {
-            if (lane == 0) lp_finish<O, E, W>(a, i, best, 0, 0, filter_ratio, false);
+            if (lane == 0) gain = a.save_gain[i];
         } else {
             part_t p = a.part[i];
             best = NO_MOVE;
             W b_conn = 0, p_conn = 0;
-            const Slot<W>* base = a.slots + a.coff[i];
-            part_t sz = a.csize[i];
-            for (part_t s = lane; s < sz; s += 32) {
-                Slot<W> sl = base[s];
+            scan_slots_part<W>(a.slots + a.coff[i], a.csize[i], lane, 32, [&](const Slot<W>& sl) {
                 if (sl.p != p) { if (lp_better<W>(sl.v, sl.p, b_conn, best)) { best = sl.p; b_conn = sl.v; } }
                 else if (sl.v > 0) p_conn = sl.v;
-            }
+            });
             for (int m = 16; m > 0; m >>= 1) {
                 W c2 = shfl_xor(b_conn, m, 32);
                 part_t e2 = shfl_xor(best, m, 32);
@@ -854,18 +1019,16 @@ __device__ __forceinline__ void d_lp_select_warp(RefArgs<O, E, W> a, const O* li
                 W pc2 = shfl_xor(p_conn, m, 32);
                 if (pc2 > p_conn) p_conn = pc2;
             }
-            if (lane == 0) lp_finish<O, E, W>(a, i, best, b_conn, p_conn, filter_ratio, true);
+            if (lane == 0) gain = lp_finish<O, E, W>(a, i, best, b_conn, p_conn, filter_ratio);
         }
-        __syncwarp();
         if (lane == 0) {
-            best = a.dest[i];
-            bool cand = best != NO_MOVE && a.lock[i] == 0;
+            const bool cand = best != NO_MOVE && lk == 0;
+            a.pregain[i] = cand ? gain : GAIN_MIN;
             if (cand) {
-                a.pregain[i] = a.save_gain[i];
+                a.dest[i] = best;
                 O s = atomic_add(&a.dev->ncand, (O)1);
                 a.cand[s] = i;
-            } else {
-                a.pregain[i] = GAIN_MIN;
+            } else if (lk) {
                 a.lock[i] = 0;
             }
         }
@@ -1065,6 +1228,60 @@ __device__ __forceinline__ void d_weak_prep(RefArgs<O, E, W> a, RebArgs<O, W> rb
 template <class O, class E, class W>
 __global__ void __launch_bounds__(1024) k_weak_prep(RefArgs<O, E, W> a, RebArgs<O, W> rb) { d_weak_prep<O, E, W>(a, rb); }
 
+// The rebalance selections' pass over every vertex: those of parts above
+// the bound that `eligible` admits have their tables scanned (`score`, with
+// the lanes PassDeal gives them); the rest get no bucket.
+template <class O, class E, class W, class Elig, class Score>
+__device__ __forceinline__ void reb_vertex_pass(const RefArgs<O, E, W>& a, const RebArgs<O, W>& rb, uint8_t* list, Elig&& eligible, Score&& score) {
+    const int lane = threadIdx.x & 31;
+    const unsigned before = (1u << lane) - 1;
+    uint8_t* sel = list + (threadIdx.x >> 5) * PASS_LIST;
+    const WarpPass wp((int64_t)a.g.n, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+    for (int64_t r = 0; r < wp.rounds; r++) {
+        const int64_t b0 = wp.base(r);
+        const int cnt = wp.count(b0);
+        if (cnt == 0) break;
+        bool in[PASS_U], heavy[PASS_U];
+        part_t p[PASS_U];
+        W sp[PASS_U];
+#pragma unroll
+        for (int u = 0; u < PASS_U; u++) {
+            const int64_t i = b0 + u * 32 + lane;
+            in[u] = u * 32 + lane < cnt;
+            p[u] = in[u] ? a.part[i] : 0;
+            if (a.mixed && in[u]) in[u] = a.g.row[i + 1] - a.g.row[i] <= THREAD_DEG;
+        }
+#pragma unroll
+        for (int u = 0; u < PASS_U; u++) sp[u] = in[u] ? a.sizes[p[u]] : (W)0;
+#pragma unroll
+        for (int u = 0; u < PASS_U; u++) heavy[u] = in[u] && sp[u] > rb.size_max && eligible((O)(b0 + u * 32 + lane), sp[u]);
+        int nh = 0;
+#pragma unroll
+        for (int u = 0; u < PASS_U; u++) {
+            const unsigned hm = __ballot_sync(0xffffffffu, heavy[u]);
+            if (heavy[u]) sel[nh + __popc(hm & before)] = (uint8_t)(u * 32 + lane);
+            else if (in[u]) rb.bid[b0 + u * 32 + lane] = -1;
+            nh += __popc(hm);
+        }
+        __syncwarp();
+        const PassDeal d(nh, lane);
+        for (int x0 = 0; x0 < nh; x0 += d.per) {
+            const bool act = x0 + d.slot < nh;
+            O i = 0;
+            part_t pi = 0, sz = 0;
+            const Slot<W>* base = nullptr;
+            if (act) {
+                i = (O)(b0 + sel[x0 + d.slot]);
+                pi = a.part[i];
+                base = a.slots + a.coff[i];
+                sz = a.csize[i];
+            }
+            score(d, act, i, pi, base, sz);
+        }
+        __syncwarp();
+    }
+}
+
 // Destination choice and bucket score (src/jet_refiner.hpp:599-645), one
 // thread per vertex (tables of vertices with deg > 32 are scanned by a warp).
 template <class O, class E, class W>
@@ -1079,8 +1296,8 @@ __device__ __forceinline__ void weak_score(const RefArgs<O, E, W>& a, const RebA
             if (tu > 0) { dest = rb.undersized[(int64_t)i % tu]; sg = -p_gain; }
         }
     }
-    a.dest[i] = dest;
     if (dest != p) {
+        a.dest[i] = dest;
         int gt = gain_bucket<W>(sg, a.g.vw[i]);
         O gid = (MAX_BUCKETS * (O)p + gt) * rb.sections + (O)(i % rb.sections);
         rb.bid[i] = gid;
@@ -1114,7 +1331,32 @@ __device__ __forceinline__ void d_weak_select_thread(RefArgs<O, E, W> a, RebArgs
     }
 }
 template <class O, class E, class W>
-__global__ void __launch_bounds__(BLOCK) k_weak_select_thread(RefArgs<O, E, W> a, RebArgs<O, W> rb) { d_weak_select_thread<O, E, W>(a, rb); }
+__device__ __forceinline__ void d_weak_select_pass(RefArgs<O, E, W> a, RebArgs<O, W> rb, uint8_t* list) {
+    reb_vertex_pass<O, E, W>(a, rb, list, [&](O i, W sp) { return (double)a.g.vw[i] < 1.5 * (double)(sp - rb.opt); },
+        [&](const PassDeal& d, bool act, O i, part_t p, const Slot<W>* base, part_t sz) {
+            W gain = 0, p_gain = 0;
+            part_t best = p;
+            scan_slots_part<W>(base, sz, d.sub, d.g, [&](const Slot<W>& sl) {
+                if (sl.p > NULL_PART && a.sizes[sl.p] < rb.max_dest) {
+                    if (sl.v > gain || (sl.v == gain && sl.v > 0 && sl.p < best)) { best = sl.p; gain = sl.v; }
+                }
+                if (sl.p == p) p_gain = sl.v;
+            });
+            for (int m = d.g >> 1; m > 0; m >>= 1) {
+                const W g2 = shfl_xor(gain, m, 32);
+                const part_t b2 = shfl_xor(best, m, 32);
+                if (g2 > gain || (g2 == gain && g2 > 0 && b2 < best)) { gain = g2; best = b2; }
+                const W pg2 = shfl_xor(p_gain, m, 32);
+                if (pg2 != 0) p_gain = pg2;
+            }
+            if (act && d.sub == 0) weak_score<O, E, W>(a, rb, i, p, best, gain, p_gain, true);
+        });
+}
+template <class O, class E, class W>
+__global__ void __launch_bounds__(BLOCK) k_weak_select_thread(RefArgs<O, E, W> a, RebArgs<O, W> rb) {
+    __shared__ uint8_t list[BLOCK / 32 * PASS_LIST];
+    d_weak_select_pass<O, E, W>(a, rb, list);
+}
 
 template <class O, class E, class W>
 __device__ __forceinline__ void d_weak_select_warp(RefArgs<O, E, W> a, RebArgs<O, W> rb, const O* list, O count) {
@@ -1226,7 +1468,37 @@ __device__ __forceinline__ void d_strong_score_thread(RefArgs<O, E, W> a, RebArg
     }
 }
 template <class O, class E, class W>
-__global__ void __launch_bounds__(BLOCK) k_strong_score_thread(RefArgs<O, E, W> a, RebArgs<O, W> rb) { d_strong_score_thread<O, E, W>(a, rb); }
+__device__ __forceinline__ void d_strong_score_pass(RefArgs<O, E, W> a, RebArgs<O, W> rb, uint8_t* list) {
+    const bool room = a.dev->total_undersized != 0;  // some part lies below max_dest
+    const W mv = a.dev->max_vwgt;
+    reb_vertex_pass<O, E, W>(a, rb, list,
+        [&](O i, W sp) {
+            const W w = a.g.vw[i];
+            return room && w <= 2 * mv && w < 2 * (sp - rb.opt);
+        },
+        [&](const PassDeal& d, bool act, O i, part_t p, const Slot<W>* base, part_t sz) {
+            uint64_t tk = 0, tg = 0;
+            W p_gain = 0;
+            scan_slots_part<W>(base, sz, d.sub, d.g, [&](const Slot<W>& sl) {
+                if (sl.p == p) p_gain = sl.v;
+                else if (sl.p > NULL_PART && a.sizes[sl.p] < rb.max_dest) { tg += (uint64_t)sl.v; tk += 1; }
+            });
+            for (int m = d.g >> 1; m > 0; m >>= 1) {
+                tg += shfl_xor(tg, m, 32);
+                tk += shfl_xor(tk, m, 32);
+                p_gain += shfl_xor(p_gain, m, 32);  // own part appears in at most one slot
+            }
+            if (act && d.sub == 0) {
+                rb.bid[i] = -1;
+                strong_score<O, E, W>(a, rb, i, p, tg, tk, p_gain);
+            }
+        });
+}
+template <class O, class E, class W>
+__global__ void __launch_bounds__(BLOCK) k_strong_score_thread(RefArgs<O, E, W> a, RebArgs<O, W> rb) {
+    __shared__ uint8_t list[BLOCK / 32 * PASS_LIST];
+    d_strong_score_pass<O, E, W>(a, rb, list);
+}
 
 template <class O, class E, class W>
 __device__ __forceinline__ void d_strong_score_warp(RefArgs<O, E, W> a, RebArgs<O, W> rb, const O* list, O count) {
@@ -1578,6 +1850,65 @@ __device__ __forceinline__ void d_reb_classify(RefArgs<O, E, W> a, RebArgs<O, W>
     }
 }
 
+// The same with PASS_U vertices per lane in flight and one append per warp
+// and list (the grid kernel).
+template <bool STRONG, class O, class E, class W>
+__device__ __forceinline__ void d_reb_classify_pass(RefArgs<O, E, W> a, RebArgs<O, W> rb, int64_t start, int64_t stride) {
+    const int lane = threadIdx.x & 31;
+    const unsigned before = (1u << lane) - 1;
+    const WarpPass wp((int64_t)a.g.n, start, stride);
+    for (int64_t r = 0; r < wp.rounds; r++) {
+        const int64_t b0 = wp.base(r);
+        const int cnt = wp.count(b0);
+        if (cnt == 0) break;
+        O b[PASS_U];
+        part_t p[PASS_U];
+        W w[PASS_U], base[PASS_U], tot[PASS_U], limit[PASS_U];
+#pragma unroll
+        for (int u = 0; u < PASS_U; u++) b[u] = u * 32 + lane < cnt ? rb.bid[b0 + u * 32 + lane] : (O)-1;
+#pragma unroll
+        for (int u = 0; u < PASS_U; u++) {
+            p[u] = b[u] >= 0 ? a.part[b0 + u * 32 + lane] : 0;
+            w[u] = b[u] >= 0 ? a.g.vw[b0 + u * 32 + lane] : (W)0;
+            tot[u] = !STRONG && b[u] >= 0 ? rb.buckets[b[u]] : (W)0;
+        }
+#pragma unroll
+        for (int u = 0; u < PASS_U; u++) {
+            base[u] = b[u] >= 0 ? rb.boff[b[u]] - rb.boff[(O)p[u] * rb.width] : (W)0;
+            limit[u] = b[u] >= 0 ? a.sizes[p[u]] - rb.size_max : (W)0;
+        }
+        int nt = 0, no = 0, at[PASS_U];  // at: the place among the warp's moves or among its queued vertices
+        bool take[PASS_U], order[PASS_U];
+#pragma unroll
+        for (int u = 0; u < PASS_U; u++) {
+            take[u] = order[u] = false;
+            if (b[u] >= 0) {
+                if ((!STRONG && b[u] >= (O)p[u] * rb.width + rb.width) || w[u] < 0) {
+                    atomicOr(&a.dev->reb_fb, 1);
+                } else if (base[u] < limit[u]) {
+                    if (!STRONG && base[u] + tot[u] < limit[u]) take[u] = true;
+                    else order[u] = true;
+                }
+            }
+            const unsigned tm = __ballot_sync(0xffffffffu, take[u]), om = __ballot_sync(0xffffffffu, order[u]);
+            at[u] = take[u] ? nt + __popc(tm & before) : no + __popc(om & before);
+            nt += __popc(tm);
+            no += __popc(om);
+        }
+        if (nt == 0 && no == 0) continue;
+        O ft = 0, fo = 0;
+        if (lane == 0 && nt) ft = atomic_add(&a.dev->nmoves, (O)nt);
+        if (lane == 0 && no) fo = atomic_add(&a.dev->nord, (O)no);
+        ft = __shfl_sync(0xffffffffu, ft, 0);
+        fo = __shfl_sync(0xffffffffu, fo, 0);
+#pragma unroll
+        for (int u = 0; u < PASS_U; u++) {
+            if (take[u]) a.moves[ft + at[u]] = (O)(b0 + u * 32 + lane);
+            if (order[u]) rb.ordl[fo + at[u]] = (O)(b0 + u * 32 + lane);
+        }
+    }
+}
+
 // Inclusive sum of v over runs that begin where head is set, across the
 // block (every thread calls it, one value each).  carry is the sum of the
 // run left open by the previous call and is updated for the next call.
@@ -1694,7 +2025,7 @@ __device__ __forceinline__ void d_reb_queue_tail(RefArgs<O, E, W> a, RebArgs<O, 
 
 template <bool STRONG, class O, class E, class W>
 __global__ void __launch_bounds__(BLOCK) k_reb_classify(RefArgs<O, E, W> a, RebArgs<O, W> rb) {
-    d_reb_classify<STRONG, O, E, W>(a, rb, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+    d_reb_classify_pass<STRONG, O, E, W>(a, rb, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
 
 // One block of 1024 threads after k_reb_classify.  When the queue fits `cap`

@@ -136,6 +136,7 @@ struct Refiner {
         a.moves_hub = moves_hub.p; a.dev = dev.p; a.filter = &ctl.p->filter;
         a.narrow = narrow_state > 0 ? 1 : 0;
         a.tw = table_width(L);
+        a.mixed = (L.n_warp > 0 || L.n_hub > 0) ? 1 : 0;
         a.pclk = phase_clk_ptr();
         return a;
     }
