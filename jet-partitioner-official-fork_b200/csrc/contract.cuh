@@ -372,17 +372,29 @@ __global__ void __launch_bounds__(THREADS) k_contract_smem(GView<O, E, W> g, con
 // shared-memory array indexed by id, then writes the nonzero entries in id
 // order (edge weights are positive, so a nonzero sum marks a neighbour).
 // Rows come out sorted with no hashing and no sort; the cost is one read of
-// the row's edges per chunk.
+// the row's edges per chunk and one sweep of the array.  The sweep was most of
+// it (a clearing pass, then a block scan with three barriers per 1024 ids):
+// now each warp owns a stretch of the array, counts its entries with 16-byte
+// reads, and after one exchange of the counts ranks them by ballots, writes
+// them and clears what it read, so the array is zero for the next chunk.
+// Edges go four per thread with every load issued before the first use.
+// R-MAT 2^24's contractions, of which this takes the hub rows of the levels
+// up to 454,000 coarse vertices: 218 -> 189 ms.
 template <class O, class E, class W>
 __global__ void __launch_bounds__(1024) k_contract_dense(GView<O, E, W> g, const O* map, const O* list, const O* count,
                                                          const O* moff, const O* members, const E* hrow, O nc, int chunk,
                                                          O* skey, W* sval, O* ucnt, int narrow) {
     extern __shared__ __align__(16) unsigned char ct_smem[];
-    W* acc = (W*)ct_smem;
+    W* acc = (W*)ct_smem;  // `chunk` (a multiple of 1024) ids
     __shared__ E s_pref[1024];
     __shared__ O s_mem[1024];
-    __shared__ int s_sw[32];
+    __shared__ int s_cnt[32];
+    constexpr int V = 16 / (int)sizeof(W);
+    struct alignas(16) Vec { W x[V]; };
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned before = (1u << lane) - 1;
     O total_rows = *count;
+    for (int i = threadIdx.x; i < chunk; i += blockDim.x) acc[i] = 0;
     for (O x = blockIdx.x; x < total_rows; x += gridDim.x) {
         O c = list[x];
         const O m0 = moff[c], m1 = moff[c + 1];
@@ -390,32 +402,80 @@ __global__ void __launch_bounds__(1024) k_contract_dense(GView<O, E, W> g, const
         for (O base = 0; base < nc; base += chunk) {
             const O top = nc - base < (O)chunk ? nc : base + chunk;
             const int len = (int)(top - base);
-            for (int i = threadIdx.x; i < len; i += blockDim.x) acc[i] = 0;
             __syncthreads();
-            auto add = [&](E j) {
-                O u = map[g.adj[j]];
-                if (u != c && u >= base && u < top) acc_add<W>(&acc[u - base], g.val[j], narrow);
-            };
             if (m1 - m0 <= 32) {
                 // few members (the usual case for dense rows): stride over each member's edges
                 for (O mi = m0; mi < m1; mi++) {
                     O i = members[mi];
-                    for (E j = g.row[i] + threadIdx.x; j < g.row[i + 1]; j += blockDim.x) add(j);
+                    const E re = g.row[i + 1];
+                    for (E j0 = g.row[i] + threadIdx.x; j0 < re; j0 += 4 * (E)blockDim.x) {
+                        O u[4];
+                        W w[4];
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const E j = j0 + q * (E)blockDim.x;
+                            u[q] = j < re ? g.adj[j] : (O)-1;
+                            w[q] = j < re ? g.val[j] : (W)0;
+                        }
+#pragma unroll
+                        for (int q = 0; q < 4; q++) u[q] = u[q] >= 0 ? map[u[q]] : c;
+#pragma unroll
+                        for (int q = 0; q < 4; q++)
+                            if (u[q] != c && u[q] >= base && u[q] < top) acc_add<W>(&acc[u[q] - base], w[q], narrow);
+                    }
                 }
             } else {
-                cta_for_row_edges<1024>(g, members, m0, m1, s_pref, s_mem, add);
+                cta_for_row_edges<1024>(g, members, m0, m1, s_pref, s_mem, [&](E j) {
+                    O u = map[g.adj[j]];
+                    if (u != c && u >= base && u < top) acc_add<W>(&acc[u - base], g.val[j], narrow);
+                });
             }
             __syncthreads();
-            // id-ordered compaction, one 1024-entry tile at a time
-            for (int t0 = 0; t0 < len; t0 += blockDim.x) {
-                int i = t0 + threadIdx.x;
-                W v = i < len ? acc[i] : (W)0;
-                int tot;
-                int ex = block_exclusive_scan<int>(v != 0 ? 1 : 0, s_sw, tot);
-                if (v != 0) { skey[out + ex] = base + (O)i; sval[out + ex] = v; }
-                out += tot;
+            // (len rounded up to a warp's step stays inside the chunk, and
+            // the ids past len hold zero)
+            constexpr int STEP = 32 * V;
+            const int steps = (len + STEP - 1) / STEP, per = (steps + 31) / 32;
+            const int lo = wid * per * STEP, hi = min((wid + 1) * per, steps) * STEP;
+            int cnt = 0;
+            for (int i = lo + lane * V; i < hi; i += STEP) {
+                const Vec v = *(const Vec*)(acc + i);
+#pragma unroll
+                for (int e = 0; e < V; e++) cnt += v.x[e] != 0;
             }
+            cnt = group_sum<int>(cnt, 32);
+            if (lane == 0) s_cnt[wid] = cnt;
             __syncthreads();
+            const int theirs = s_cnt[lane];
+            E pos = out + (E)group_sum<int>(lane < wid ? theirs : 0, 32);
+            out += (E)group_sum<int>(theirs, 32);
+            if (cnt) {
+                for (int i = lo + lane * V; i < hi; i += STEP) {
+                    const Vec v = *(const Vec*)(acc + i);
+                    int rank = 0, all = 0;
+                    bool any = false;
+#pragma unroll
+                    for (int e = 0; e < V; e++) {
+                        const unsigned m = __ballot_sync(0xffffffffu, v.x[e] != 0);
+                        rank += __popc(m & before);
+                        all += __popc(m);
+                    }
+#pragma unroll
+                    for (int e = 0; e < V; e++) {
+                        if (v.x[e] == 0) continue;
+                        skey[pos + rank] = base + (O)(i + e);
+                        sval[pos + rank] = v.x[e];
+                        rank++;
+                        any = true;
+                    }
+                    if (any) {
+                        Vec z;
+#pragma unroll
+                        for (int e = 0; e < V; e++) z.x[e] = 0;
+                        *(Vec*)(acc + i) = z;
+                    }
+                    pos += all;
+                }
+            }
         }
         if (threadIdx.x == 0) ucnt[c] = (O)(out - hrow[c]);
         __syncthreads();

@@ -426,6 +426,9 @@ struct Engine {
         // takes at most DENSE_PASSES chunks, else (row, neighbour) keys + radix sort
         int dense_chunk = (max_dynamic_smem((const void*)k_contract_dense<O, E, W>) - 1024) / (int)sizeof(W);
         dense_chunk &= ~1023;
+        // no more than the ids there are, so that two blocks share an SM on
+        // levels of up to about 27,000 coarse vertices (32-bit weights)
+        if ((int64_t)nc < (int64_t)dense_chunk) dense_chunk = ((int)nc + 1023) & ~1023;
         const bool dense = dense_chunk > 0 && (int64_t)nc <= (int64_t)DENSE_PASSES * dense_chunk;
         if (dense)
             JET_CUDA(cudaFuncSetAttribute(k_contract_dense<O, E, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -492,7 +495,9 @@ struct Engine {
                 g, map, l2.p, n2, moff.p, members.p, hrow.p, skey, sval, ucnt.p, nc, narrow_w); count_launch();
             JET_LAUNCH_CHECK();
             if (dense) {
-                k_contract_dense<O, E, W><<<device_info().sms, 1024, (size_t)dense_chunk * sizeof(W), s>>>(
+                JET_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_contract_dense<O, E, W>, 1024,
+                                                                       (size_t)dense_chunk * sizeof(W)));
+                k_contract_dense<O, E, W><<<device_info().sms * (per_sm > 0 ? per_sm : 1), 1024, (size_t)dense_chunk * sizeof(W), s>>>(
                     g, map, lh.p, nh, moff.p, members.p, hrow.p, nc, dense_chunk, skey, sval, ucnt.p, narrow_w); count_launch();
                 JET_LAUNCH_CHECK();
             } else {

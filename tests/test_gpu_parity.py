@@ -226,6 +226,25 @@ def _skewed_runs(jet, orc, g, og, k, imb, skew, iters_list=(1, 2, 3, 6, 10)):
     return seen
 
 
+@pytest.mark.parametrize("n", [8192, 8194, 8450, 130001], ids=["whole_steps", "one_over", "one_step_over", "two_or_more_chunks"])
+@pytest.mark.parametrize("tier", TIERS)
+def test_contract_dense_rows(jet, graphs, orc, tier, n):
+    """Hub rows through the dense accumulator: coarse id counts at and just
+    past a multiple of a warp's sweep step (128 ids in 32 bits, 64 in 64) and
+    past one chunk of the array; rows that touch every id and a few."""
+    gen = torch.Generator().manual_seed(n)
+    far = torch.randint(n // 2, n, (4200,), generator=gen)
+    u = torch.cat([torch.zeros(n - 1, dtype=torch.long), torch.full((4200,), 2), torch.arange(3, n - 1)])
+    v = torch.cat([torch.arange(1, n), far, torch.arange(4, n)])
+    g = graphs.from_undirected(n, u, v, torch.randint(1, 9, (u.numel(),), generator=gen)).as_tier(tier)
+    m = (np.arange(n) // 2).astype(np.int64 if tier == "biggest" else np.int32)
+    nc = (n + 1) // 2
+    want = orc.contract(orc.G.from_csr(g), m, nc)
+    got = jet.contract(g.to("cuda"), torch.from_numpy(m).cuda(), nc)
+    assert np.array_equal(host(got.row), want.row) and np.array_equal(host(got.adj), want.adj)
+    assert np.array_equal(host(got.val), want.val) and np.array_equal(host(got.vw), want.vw)
+
+
 @pytest.mark.parametrize("tier", ["i32", "big"])
 def test_rebalance_queue_overflow_falls_back(jet, graphs, orc, tier):
     """A 250 x 250 mesh with 90% of its vertices piled into one part: the
