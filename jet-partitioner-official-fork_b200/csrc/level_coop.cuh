@@ -282,6 +282,8 @@ __device__ __forceinline__ bool coop_reb_tail(RefArgs<O, E, W>& a, RebArgs<O, W>
         pc.mark(PH_STRONG_FIRST);
         if (blockIdx.x == 0) d_strong_redraw<O, E, W>(a, rb);
         if (!level_sync<CL>(cs.bar, err)) return false;
+        d_strong_gain<O, E, W>(a, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+        if (!level_sync<CL>(cs.bar, err)) return false;
         pc.mark(PH_REDRAW);
     }
     return true;
@@ -298,7 +300,15 @@ k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O,
              W* sizes_best, CoopScratch<O, E, W> cs, int bits, int max_iters) {
     int* err = &a.dev->err;
     const O n = a.g.n;
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl_begin_logic(c);
+    __shared__ int s_mode;  // of the next iteration, in the block that prepares it
+    if (blockIdx.x == 0) {
+        if (threadIdx.x == 0) {
+            ctl_begin_logic(c);
+            s_mode = c->mode;
+        }
+        __syncthreads();
+        next_prep<O, E, W>(a, rbw, rbs, s_mode);
+    }
     if (!level_sync<CL>(cs.bar, err)) return;
     PhaseClock pc(a.pclk, CL ? 2 * PHASE_SLOTS : 4 * PHASE_SLOTS, blockIdx.x == 0 && threadIdx.x == 0);
     while (true) {
@@ -326,15 +336,6 @@ k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O,
             }
         } else {
             RebArgs<O, W>& rb = mode == MODE_WEAK ? rbw : rbs;
-            // bucket totals cleared while block 0 lists the parts (neither
-            // reads what the other writes)
-            coop_zero<O, E, W>(rb.buckets, (int64_t)rb.t_minibuckets + 1 + rb.width);
-            if (blockIdx.x == 0) {
-                if (mode == MODE_WEAK) d_weak_prep<O, E, W>(a, rb);
-                else d_strong_prep<O, E, W>(a, rb);
-            }
-            if (!level_sync<CL>(cs.bar, err)) return;
-            pc.mark(PH_REB_PREP);
             if (mode == MODE_WEAK) {
                 d_weak_select_thread<O, E, W>(a, rb);
                 d_weak_select_warp<O, E, W>(a, rb, li.warp_list, li.n_warp);
@@ -351,29 +352,20 @@ k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O,
             if (!ok) return;
         }
         // perform_moves (src/jet_refiner.hpp:905-955)
-        d_apply_moves<O, E, W>(a, 0);
+        d_apply_moves<O, E, W>(a, li.group);
+        if (mode != MODE_LP)  // for the next rebalance: the last one is done with them
+            coop_zero<O, E, W>(rbw.buckets, (int64_t)rbw.t_minibuckets + 1 + rbw.width);
         if (!level_sync<CL>(cs.bar, err)) return;
         pc.mark(PH_APPLY);
-        switch (li.group) {
-            case 4: d_update_small<4, false, O, E, W>(a); break;
-            case 8: d_update_small<8, false, O, E, W>(a); break;
-            case 16: d_update_small<16, false, O, E, W>(a); break;
-            default: d_update_small<32, false, O, E, W>(a); break;
+        if (li.n_hub > 0) {
+            d_apply_hub<O, E, W>(a);
+            if (!level_sync<CL>(cs.bar, err)) return;
+            pc.mark(PH_UPDATE_SUB);
         }
-        d_update_small_hub<false, O, E, W>(a);
-        if (!level_sync<CL>(cs.bar, err)) return;
-        pc.mark(PH_UPDATE_SUB);
-        switch (li.group) {
-            case 4: d_update_small<4, true, O, E, W>(a); d_mark_neighbors<4, O, E, W>(a); break;
-            case 8: d_update_small<8, true, O, E, W>(a); d_mark_neighbors<8, O, E, W>(a); break;
-            case 16: d_update_small<16, true, O, E, W>(a); d_mark_neighbors<16, O, E, W>(a); break;
-            default: d_update_small<32, true, O, E, W>(a); d_mark_neighbors<32, O, E, W>(a); break;
-        }
-        d_update_small_hub<true, O, E, W>(a);
-        d_mark_neighbors_hub<O, E, W>(a);
-        if (!level_sync<CL>(cs.bar, err)) return;
-        pc.mark(PH_UPDATE_ADD);
-        if (a.dev->large) {
+        if (!ld_cg(&a.dev->large)) {
+            d_update_add<O, E, W>(a, li.group);
+            if (li.n_hub > 0) d_update_add_hub<O, E, W>(a);
+        } else {
             // update_large: queue the marked rows (one coalesced pass), then
             // rebuild them one warp per row
             for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
@@ -385,33 +377,24 @@ k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O,
             if (!level_sync<CL>(cs.bar, err)) return;
             d_conn_warp<O, E, W>(a, cs.marked, (O)((volatile GridBar*)cs.bar)->nmarked, 1, nullptr);
             if (!level_sync<CL>(cs.bar, err)) return;
+            pc.mark(PH_REBUILD);
+            d_cut_after<O, E, W>(a);
         }
-        pc.mark(PH_REBUILD);
-        d_cut_after<O, E, W>(a);
-        // the last block to finish its share of the cut change closes the
-        // iteration (one barrier instead of two): its fence and counter add
-        // come after every other block's cut atomics
-        {
-            __shared__ int s_last;
-            __syncthreads();
+        // the last block to get here closes the iteration (one barrier less):
+        // its fence and counter add come after every other block's atomics
+        if (last_block(&cs.bar->cut_done)) {
+            W mx = block_max_sizes<W>(a.sizes, a.k);
             if (threadIdx.x == 0) {
-                __threadfence();
-                s_last = atomicAdd(&cs.bar->cut_done, 1u) == gridDim.x - 1;
+                ctl_end_logic<O, W>(c, a.dev, mx);
+                cs.bar->nmarked = 0;
+                if (c->more && c->iter_count >= max_iters) { c->more = 0; atomicOr(err, ERRF_SPIN); }
+                s_mode = c->more ? c->mode : MODE_LP;
             }
             __syncthreads();
-            if (s_last) {
-                __threadfence();
-                W mx = block_max_sizes<W>(a.sizes, a.k);
-                if (threadIdx.x == 0) {
-                    cs.bar->cut_done = 0;
-                    ctl_end_logic<O, W>(c, a.dev, mx);
-                    cs.bar->nmarked = 0;
-                    if (c->more && c->iter_count >= max_iters) { c->more = 0; atomicOr(err, ERRF_SPIN); }
-                }
-            }
+            next_prep<O, E, W>(a, rbw, rbs, s_mode);
         }
         if (!level_sync<CL>(cs.bar, err)) return;
-        pc.mark(PH_CUT);
+        pc.mark(PH_UPDATE_ADD);
         // the copy of the best state needs no barrier of its own: what it
         // reads (parts, sizes) is next written by the apply phase, at least
         // one barrier later, and nothing reads what it writes during the loop

@@ -190,6 +190,8 @@ __device__ __forceinline__ void d_reb_tail(RefArgs<O, E, W> a, RebArgs<O, W> rb,
         pc.mark(PH_STRONG_FIRST);
         d_strong_redraw<O, E, W>(a, rb);
         __syncthreads();
+        d_strong_gain<O, E, W>(a, threadIdx.x, blockDim.x);
+        __syncthreads();
         pc.mark(PH_REDRAW);
     }
 }
@@ -198,7 +200,6 @@ template <class O, class E, class W>
 __device__ __forceinline__ void cta_zero_buckets(const RebArgs<O, W>& rb) {
     int64_t m = (int64_t)rb.t_minibuckets + 1 + rb.width;
     for (int64_t i = threadIdx.x; i < m; i += blockDim.x) rb.buckets[i] = 0;
-    __syncthreads();
 }
 
 // Where the single-CTA loop keeps the level's mutable state.  The loop is
@@ -209,7 +210,7 @@ __device__ __forceinline__ void cta_zero_buckets(const RebArgs<O, W>& rb) {
 // launch touches these arrays, so moving them cannot change a result.
 static constexpr uint32_t NO_SMEM = 0xffffffffu;
 struct CtaSmemPlan {
-    uint32_t part, dest, csize, dest_cache, save_gain, pregain, lock, mark;
+    uint32_t part, dest, csize, dest_cache, save_gain, pregain, lock, mark, stamp;
     uint32_t cand, moves, bid, score, sizes, dev, ctl, slots, buckets, boff;
     int64_t nslots, nbuckets;
     size_t total;  // dynamic shared memory the launch needs
@@ -244,6 +245,7 @@ k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, 
         cta_place(smem_raw, plan.pregain, a.pregain, n);
         cta_place(smem_raw, plan.lock, a.lock, n);
         cta_place(smem_raw, plan.mark, a.mark, n);
+        cta_place(smem_raw, plan.stamp, a.stamp, n);
         cta_place(smem_raw, plan.cand, a.cand, n);
         cta_place(smem_raw, plan.moves, a.moves, n);
         cta_place(smem_raw, plan.sizes, a.sizes, a.k);
@@ -263,6 +265,8 @@ k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, 
         s_mode = c->mode;
         s_more = c->more;
     }
+    __syncthreads();
+    next_prep<O, E, W>(a, rbw, rbs, s_mode);
     __syncthreads();
     PhaseClock pc(a.pclk, 0, threadIdx.x == 0);
     int iters = 0;
@@ -286,10 +290,6 @@ k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, 
             __syncthreads();
             pc.mark(PH_AFTERBURN_HUB);
         } else if (mode == MODE_WEAK) {
-            cta_zero_buckets<O, E, W>(rbw);
-            d_weak_prep<O, E, W>(a, rbw);
-            __syncthreads();
-            pc.mark(PH_REB_PREP);
             d_weak_select_thread<O, E, W>(a, rbw);
             d_weak_select_warp<O, E, W>(a, rbw, li.warp_list, li.n_warp);
             d_weak_select_warp<O, E, W>(a, rbw, li.hub_list, li.n_hub);
@@ -297,10 +297,6 @@ k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, 
             pc.mark(PH_REB_SELECT);
             d_reb_tail<false, O, E, W>(a, rbw, keys, P, pc);
         } else {
-            cta_zero_buckets<O, E, W>(rbs);
-            d_strong_prep<O, E, W>(a, rbs);
-            __syncthreads();
-            pc.mark(PH_REB_PREP);
             d_strong_score_thread<O, E, W>(a, rbs);
             d_strong_score_warp<O, E, W>(a, rbs, li.warp_list, li.n_warp);
             d_strong_score_warp<O, E, W>(a, rbs, li.hub_list, li.n_hub);
@@ -309,34 +305,28 @@ k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, 
             d_reb_tail<true, O, E, W>(a, rbs, keys, P, pc);
         }
         // perform_moves (src/jet_refiner.hpp:905-955)
-        d_apply_moves<O, E, W>(a, 0);
+        d_apply_moves<O, E, W>(a, li.group);
+        if (mode != MODE_LP) cta_zero_buckets<O, E, W>(rbw);  // for the next rebalance: the last one is done with them
         __syncthreads();
         pc.mark(PH_APPLY);
-        switch (li.group) {
-            case 4: d_update_small<4, false, O, E, W>(a); break;
-            case 8: d_update_small<8, false, O, E, W>(a); break;
-            case 16: d_update_small<16, false, O, E, W>(a); break;
-            default: d_update_small<32, false, O, E, W>(a); break;
+        if (li.n_hub > 0) {
+            d_apply_hub<O, E, W>(a);
+            __syncthreads();
+            pc.mark(PH_UPDATE_SUB);
         }
-        d_update_small_hub<false, O, E, W>(a);
-        __syncthreads();
-        pc.mark(PH_UPDATE_SUB);
-        switch (li.group) {
-            case 4: d_update_small<4, true, O, E, W>(a); d_mark_neighbors<4, O, E, W>(a); break;
-            case 8: d_update_small<8, true, O, E, W>(a); d_mark_neighbors<8, O, E, W>(a); break;
-            case 16: d_update_small<16, true, O, E, W>(a); d_mark_neighbors<16, O, E, W>(a); break;
-            default: d_update_small<32, true, O, E, W>(a); d_mark_neighbors<32, O, E, W>(a); break;
+        if (!a.dev->large) {
+            d_update_add<O, E, W>(a, li.group);
+            if (li.n_hub > 0) d_update_add_hub<O, E, W>(a);
+            __syncthreads();
+            pc.mark(PH_UPDATE_ADD);
+        } else {
+            d_conn_warp<O, E, W>(a, nullptr, n, 1, nullptr);  // update_large: rebuild the marked rows
+            __syncthreads();
+            pc.mark(PH_REBUILD);
+            d_cut_after<O, E, W>(a);
+            __syncthreads();
+            pc.mark(PH_CUT);
         }
-        d_update_small_hub<true, O, E, W>(a);
-        d_mark_neighbors_hub<O, E, W>(a);
-        __syncthreads();
-        pc.mark(PH_UPDATE_ADD);
-        d_conn_warp<O, E, W>(a, nullptr, n, 1, &a.dev->large);  // update_large: rebuild marked rows
-        __syncthreads();
-        pc.mark(PH_REBUILD);
-        d_cut_after<O, E, W>(a);
-        __syncthreads();
-        pc.mark(PH_CUT);
         W mx = block_max_sizes<W>(a.sizes, a.k);
         if (threadIdx.x == 0) {
             ctl_end_logic<O, W>(c, a.dev, mx);
@@ -346,6 +336,7 @@ k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, 
             if (c->more && iters >= max_iters) atomicOr(&a.dev->err, ERRF_SPIN);
         }
         __syncthreads();
+        next_prep<O, E, W>(a, rbw, rbs, s_mode);  // (the copy below reads neither list)
         pc.mark(PH_CTL);
         if (s_copy) {
             for (int64_t i = threadIdx.x; i < n; i += blockDim.x) best_part[i] = a.part[i];
@@ -358,7 +349,10 @@ k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, 
     // the host reads the control state and the error flags after the level
     if (threadIdx.x == 0) {
         if (plan.ctl != NO_SMEM) *c_global = *c;
-        if (plan.dev != NO_SMEM && a.dev->err) atomicOr(&dev_global->err, a.dev->err);
+        if (plan.dev != NO_SMEM) {
+            if (a.dev->err) atomicOr(&dev_global->err, a.dev->err);
+            dev_global->iter = a.dev->iter;  // stamps of later levels must not repeat these
+        }
     }
 }
 
@@ -368,7 +362,7 @@ template <class O, class W>
 inline CtaSmemPlan plan_cta_smem(int64_t n, int64_t nslots, int64_t nbuckets, int k, size_t scratch, size_t budget,
                                  bool enable) {
     CtaSmemPlan pl;
-    uint32_t* fields[] = {&pl.part, &pl.dest, &pl.csize, &pl.dest_cache, &pl.save_gain, &pl.pregain, &pl.lock, &pl.mark,
+    uint32_t* fields[] = {&pl.part, &pl.dest, &pl.csize, &pl.dest_cache, &pl.save_gain, &pl.pregain, &pl.lock, &pl.mark, &pl.stamp,
                           &pl.cand, &pl.moves, &pl.bid, &pl.score, &pl.sizes, &pl.dev, &pl.ctl, &pl.slots,
                           &pl.buckets, &pl.boff};
     for (uint32_t* f : fields) *f = NO_SMEM;
@@ -401,6 +395,7 @@ inline CtaSmemPlan plan_cta_smem(int64_t n, int64_t nslots, int64_t nbuckets, in
     take(pl.score, n * sizeof(W));
     take(pl.buckets, nbuckets * sizeof(W));
     take(pl.boff, nbuckets * sizeof(W));
+    take(pl.stamp, n * sizeof(uint32_t));
     pl.total = off;
     return pl;
 }

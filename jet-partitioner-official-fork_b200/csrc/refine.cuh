@@ -78,6 +78,7 @@ struct RefDev {
     part_t total_undersized;
     int err;
     int large;            // this iteration used update_large
+    uint32_t iter;        // iterations closed so far; the running one stamps its moves iter + 1
     O nord;               // rebalance: candidates queued for in-bucket ordering
     O nord_last;          // (their count in the last rebalance, for profiling)
     int reb_fb;           // rebalance: the queue cannot be used (fallback to the full sort)
@@ -106,7 +107,8 @@ struct RefArgs {
     part_t* part;
     part_t* dest;
     W* save_gain;
-    W* pregain;
+    W* pregain;            // LP: priority; every mode: connection gain of each move
+    uint32_t* stamp;       // iteration in which a vertex moved last (RefDev::iter)
     W* sizes;
     O* cand;
     O* cand_hub;
@@ -1215,7 +1217,7 @@ template <class O, class E, class W>
 __device__ __forceinline__ void d_weak_prep(RefArgs<O, E, W> a, RebArgs<O, W> rb) {
     __shared__ int sw[32];
     int carry = 0;
-    for (int base = 0; base < a.k; base += 1024) {
+    for (int base = 0; base < a.k; base += blockDim.x) {
         int p = base + threadIdx.x;
         int f = (p < a.k && a.sizes[p] < rb.max_dest) ? 1 : 0;
         int tot;
@@ -1298,6 +1300,7 @@ __device__ __forceinline__ void weak_score(const RefArgs<O, E, W>& a, const RebA
     }
     if (dest != p) {
         a.dest[i] = dest;
+        a.pregain[i] = sg;
         int gt = gain_bucket<W>(sg, a.g.vw[i]);
         O gid = (MAX_BUCKETS * (O)p + gt) * rb.sections + (O)(i % rb.sections);
         rb.bid[i] = gid;
@@ -1800,6 +1803,23 @@ __device__ __forceinline__ void d_strong_redraw(RefArgs<O, E, W> a, RebArgs<O, W
 template <class O, class E, class W>
 __global__ void __launch_bounds__(1024) k_strong_redraw(RefArgs<O, E, W> a, RebArgs<O, W> rb) { d_strong_redraw<O, E, W>(a, rb); }
 
+// Connection gains of the strong rebalance's moves, read from the tables
+// before any of them is updated (LP and weak selection store theirs).
+template <class O, class E, class W>
+__device__ __forceinline__ void d_strong_gain(const RefArgs<O, E, W>& a, int64_t start, int64_t stride) {
+    const O count = a.dev->nmoves;
+    for (int64_t x = start; x < count; x += stride) {
+        const O v = a.moves[x];
+        const Slot<W>* base = a.slots + a.coff[v];
+        const part_t sz = a.csize[v];
+        a.pregain[v] = table_lookup<W>(base, a.dest[v], sz, a.k) - table_lookup<W>(base, a.part[v], sz, a.k);
+    }
+}
+template <class O, class E, class W>
+__global__ void __launch_bounds__(BLOCK) k_strong_gain(RefArgs<O, E, W> a) {
+    d_strong_gain<O, E, W>(a, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+}
+
 // ---------------------------------------------------------------- eviction from a short queue
 // A candidate's eviction score (get_evictions, src/jet_refiner.hpp:392-409)
 // is the offset of its bucket inside its part's bucket range plus "within",
@@ -2019,6 +2039,8 @@ __device__ __forceinline__ void d_reb_queue_tail(RefArgs<O, E, W> a, RebArgs<O, 
         if (pc) pc->mark(PH_STRONG_FIRST);
         d_strong_redraw<O, E, W>(a, rb, (unsigned char*)keys, (size_t)key_cap * sizeof(uint64_t));
         __syncthreads();
+        d_strong_gain<O, E, W>(a, threadIdx.x, blockDim.x);
+        __syncthreads();  // the one-CTA loop goes straight on to the moves
         if (pc) pc->mark(PH_REDRAW);
     }
 }
@@ -2060,44 +2082,17 @@ __global__ void __launch_bounds__(1024) k_reb_ordered(RefArgs<O, E, W> a, RebArg
 }
 
 // ---------------------------------------------------------------- moves
-// perform_moves part 1 (src/jet_refiner.hpp:910-931): cut change from the old
-// tables, apply the moves, part-size deltas through a shared histogram.
-template <class O, class E, class W>
-__device__ __forceinline__ void d_apply_moves(RefArgs<O, E, W> a, int hist) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    W* hs = (W*)smem_raw;
-    if (hist) {
-        for (int p = threadIdx.x; p < a.k; p += blockDim.x) hs[p] = 0;
-        __syncthreads();
-    }
-    O count = a.dev->nmoves;
-    W c1 = 0;
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < count; x += stride) {
-        O i = a.moves[x];
-        part_t p = a.part[i], b = a.dest[i];
-        const Slot<W>* base = a.slots + a.coff[i];
-        part_t sz = a.csize[i];
-        c1 += table_lookup<W>(base, b, sz, a.k) - table_lookup<W>(base, p, sz, a.k);
-        a.dest_cache[i] = NULL_PART;
-        W w = a.g.vw[i];
-        if (hist) { atomic_add(&hs[p], -w); atomic_add(&hs[b], w); }
-        else { atomic_add(&a.sizes[p], -w); atomic_add(&a.sizes[b], w); }
-        a.part[i] = b;
-        a.dest[i] = p;
-        if (a.g.row[i + 1] - a.g.row[i] > HUB_DEG) { O s = atomic_add(&a.dev->nmoves_hub, (O)1); a.moves_hub[s] = i; }
-    }
-    c1 = group_sum<W>(c1, 32);
-    if ((threadIdx.x & 31) == 0 && c1) atomic_add(&a.dev->cut1, c1);
-    if (hist) {
-        __syncthreads();
-        for (int p = threadIdx.x; p < a.k; p += blockDim.x) if (hs[p]) atomic_add(&a.sizes[p], hs[p]);
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.dev->large = count > (O)(a.g.n / 10);
-}
-template <class O, class E, class W>
-__global__ void __launch_bounds__(BLOCK) k_apply_moves(RefArgs<O, E, W> a, int hist) { d_apply_moves<O, E, W>(a, hist); }
-
+// perform_moves (src/jet_refiner.hpp:905-955) in two phases. The first makes
+// the moves and takes their weights out of the neighbours' tables (or, for
+// update_large, marks the neighbours); the second adds them to the tables'
+// new parts. The cut change needs no phase of its own: a move's connection
+// gain is known from its selection, and after all moves a table differs from
+// what the gain was read from by the edges between moved vertices, which the
+// second phase meets on its way (stamp). Before, the moves, the two table
+// passes and the lookups after them were four phases with a barrier or a
+// launch each. Per iteration, before and after (128^3 mesh into 64 parts, levels
+// of 3,971 / 70,288 / 749,582 / 2.1 M vertices): 64 / 70 / 112 / 118 us, now
+// 55 / 57 / 103 / 107; a 65,536-vertex 2D mesh level in the cluster 44 -> 36.
 // update_small subtract (src/jet_refiner.hpp:786-808).
 template <class O, class E, class W>
 __device__ __forceinline__ void conn_sub(const RefArgs<O, E, W>& a, O v, part_t p, W w) {
@@ -2120,27 +2115,29 @@ __device__ __forceinline__ void conn_add(const RefArgs<O, E, W>& a, O v, part_t 
     E vs = a.coff[v];
     Slot<W>* base = a.slots + vs;
     part_t vsize = ld_cg(&a.csize[v]);
-    const part_t home = slot_home(best, vsize, a.k);
-    part_t po = home;
-    bool success = false;
-    for (part_t q = 0, pi = home; q < vsize; q++) {
-        part_t e = ld_cg(&base[pi].p);
+    // best, or the first slot that can take it: a slot seen occupied by
+    // another part stays so during this phase
+    part_t po = slot_home(best, vsize, a.k), px = best, count = 0, step = 0;
+    bool success = false, room = false;
+    for (part_t q = 0, pi = po; q < vsize; q++) {
+        const part_t e = ld_cg(&base[pi].p);
         if (e == best) { success = true; po = pi; break; }
-        else if (e == NULL_PART) break;
+        if (e <= NULL_PART && !room) { room = true; po = pi; px = e; step = q; }
+        if (e == NULL_PART) break;
         pi = pi + 1 == vsize ? 0 : pi + 1;
     }
-    part_t count = 0;
+    count = room ? step : vsize;
     while (!success && count < vsize) {
-        part_t px = ld_cg(&base[po].p);
-        while (px != best && px > NULL_PART && count++ < vsize) {
+        if (px == best) {
+            success = true;
+        } else if (px > NULL_PART) {
             po = po + 1 == vsize ? 0 : po + 1;
+            count++;
             px = ld_cg(&base[po].p);
-        }
-        if (px == best) success = true;
-        else if (px <= NULL_PART) {
-            part_t old = atomicCAS((int*)&base[po].p, px, best);
-            if (old == best || old <= NULL_PART) success = true;
-            else { po = po + 1 == vsize ? 0 : po + 1; count++; }
+        } else {
+            const part_t old = atomicCAS((int*)&base[po].p, px, best);
+            if (old == px) success = true;
+            else px = old;
         }
     }
     if (!success) {
@@ -2166,103 +2163,168 @@ __device__ __forceinline__ void conn_add(const RefArgs<O, E, W>& a, O v, part_t 
     atomic_add(&base[po].v, w);
 }
 
-template <int G, bool ADD, class O, class E, class W>
-__device__ __forceinline__ void d_update_small(RefArgs<O, E, W> a) {
-    if (a.dev->large) return;
-    O count = a.dev->nmoves;
-#define UPD_BODY(x, in, lane)                                                               \
-    {                                                                                       \
-        if (in) {                                                                           \
-            O i = a.moves[x];                                                               \
-            E s = a.g.row[i], e = a.g.row[i + 1];                                           \
-            if (e - s <= HUB_DEG) {                                                         \
-                part_t pp = ADD ? a.part[i] : a.dest[i];                                    \
-                for (E j = s + lane; j < e; j += G) {                                       \
-                    if (ADD) conn_add<O, E, W>(a, a.g.adj[j], pp, a.g.val[j]);              \
-                    else conn_sub<O, E, W>(a, a.g.adj[j], pp, a.g.val[j]);                  \
-                }                                                                           \
-            }                                                                               \
-        }                                                                                   \
-    }
-    JET_GROUP_LOOP(G, count, UPD_BODY)
-#undef UPD_BODY
-}
-template <int G, bool ADD, class O, class E, class W>
-__global__ void __launch_bounds__(BLOCK) k_update_small(RefArgs<O, E, W> a) { d_update_small<G, ADD, O, E, W>(a); }
-
-template <bool ADD, class O, class E, class W>
-__device__ __forceinline__ void d_update_small_hub(RefArgs<O, E, W> a) {
-    if (a.dev->large) return;
-    O count = a.dev->nmoves_hub;
-    for (O x = blockIdx.x; x < count; x += gridDim.x) {
-        O i = a.moves_hub[x];
-        part_t pp = ADD ? a.part[i] : a.dest[i];
-        for (E j = a.g.row[i] + threadIdx.x; j < a.g.row[i + 1]; j += blockDim.x) {
-            if (ADD) conn_add<O, E, W>(a, a.g.adj[j], pp, a.g.val[j]);
-            else conn_sub<O, E, W>(a, a.g.adj[j], pp, a.g.val[j]);
-        }
-    }
-}
-template <bool ADD, class O, class E, class W>
-__global__ void __launch_bounds__(1024) k_update_small_hub(RefArgs<O, E, W> a) { d_update_small_hub<ADD, O, E, W>(a); }
-
-// update_large (src/jet_refiner.hpp:743-777): mark every neighbour of a
-// moved vertex; the marked rows are rebuilt by the table builders.
-template <int G, class O, class E, class W>
-__device__ __forceinline__ void d_mark_neighbors(RefArgs<O, E, W> a) {
-    if (!a.dev->large) return;
-    O count = a.dev->nmoves;
-#define MARK_BODY(x, in, lane)                                                              \
-    {                                                                                       \
-        if (in) {                                                                           \
-            O i = a.moves[x];                                                               \
-            E rs = a.g.row[i], re = a.g.row[i + 1];                                         \
-            if (re - rs <= HUB_DEG)  /* hubs: one CTA each (d_mark_neighbors_hub) */         \
-                for (E j0 = rs + lane; j0 < re; j0 += 4 * G) {                              \
-                    /* four neighbours per lane, every load issued before the first use */  \
-                    O v[4];                                                                 \
-                    uint8_t mk[4];                                                          \
-                    _Pragma("unroll") for (int u = 0; u < 4; u++)                           \
-                        v[u] = j0 + (E)u * G < re ? a.g.adj[j0 + (E)u * G] : (O)-1;         \
-                    _Pragma("unroll") for (int u = 0; u < 4; u++)                           \
-                        mk[u] = v[u] >= 0 ? a.mark[v[u]] : (uint8_t)1;                      \
-                    /* read first: few lines get dirtied */                                 \
-                    _Pragma("unroll") for (int u = 0; u < 4; u++)                           \
-                        if (!mk[u]) a.mark[v[u]] = 1;                                       \
-                }                                                                           \
-        }                                                                                   \
-    }
-    JET_GROUP_LOOP(G, count, MARK_BODY)
-#undef MARK_BODY
-}
-template <int G, class O, class E, class W>
-__global__ void __launch_bounds__(BLOCK) k_mark_neighbors(RefArgs<O, E, W> a) { d_mark_neighbors<G, O, E, W>(a); }
-
+// Marks neighbours j0, j0 + stride, ... of a row for a rebuild: four per
+// round, every load issued before the first use, and only unmarked ones
+// written, so that few lines get dirty.
 template <class O, class E, class W>
-__device__ __forceinline__ void d_mark_neighbors_hub(RefArgs<O, E, W> a) {
-    if (!a.dev->large) return;
-    O count = a.dev->nmoves_hub;
+__device__ __forceinline__ void mark_edges(const RefArgs<O, E, W>& a, E j0, E re, E stride) {
+    for (; j0 < re; j0 += 4 * stride) {
+        O v[4];
+        uint8_t mk[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = j0 + (E)u * stride < re ? a.g.adj[j0 + (E)u * stride] : (O)-1;
+#pragma unroll
+        for (int u = 0; u < 4; u++) mk[u] = v[u] >= 0 ? a.mark[v[u]] : (uint8_t)1;
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (!mk[u]) a.mark[v[u]] = 1;
+    }
+}
+
+// First phase. HIST: part-size deltas gather in hs (k entries of shared
+// memory, zeroed here) and are added to the sizes at the end; else each move's
+// are added to the sizes directly.
+// Rows above HUB_DEG are only listed here; d_apply_hub walks them.
+template <int G, bool HIST, class O, class E, class W>
+__device__ __forceinline__ void d_apply_moves(const RefArgs<O, E, W>& a, W* hs) {
+    if (HIST) {
+        for (int p = threadIdx.x; p < a.k; p += blockDim.x) hs[p] = 0;
+        __syncthreads();
+    }
+    const O count = a.dev->nmoves;
+    const bool large = count > (O)(a.g.n / 10);
+    const uint32_t now = a.dev->iter + 1;
+    W c1 = 0;
+#define APPLY_BODY(x, in, lane)                                                             \
+    {                                                                                       \
+        O i = 0; E s = 0, e = 0; part_t p = 0, b = 0;                                       \
+        if (in) { i = a.moves[x]; s = a.g.row[i]; e = a.g.row[i + 1]; p = a.part[i]; b = a.dest[i]; } \
+        __syncwarp();  /* the group has read the part and destination */                    \
+        if (in && lane == 0) {                                                              \
+            const W w = a.g.vw[i];                                                          \
+            c1 += a.pregain[i];                                                             \
+            a.dest_cache[i] = NULL_PART;                                                    \
+            a.part[i] = b;                                                                  \
+            a.dest[i] = p;                                                                  \
+            a.stamp[i] = now;                                                               \
+            if (HIST) { atomic_add(&hs[p], -w); atomic_add(&hs[b], w); }                    \
+            else { atomic_add(&a.sizes[p], -w); atomic_add(&a.sizes[b], w); }               \
+            if (e - s > HUB_DEG) { O h = atomic_add(&a.dev->nmoves_hub, (O)1); a.moves_hub[h] = i; } \
+        }                                                                                   \
+        if (in && e - s <= HUB_DEG) {                                                       \
+            if (large) mark_edges<O, E, W>(a, s + lane, e, (E)G);                           \
+            else for (E j = s + lane; j < e; j += G) conn_sub<O, E, W>(a, a.g.adj[j], p, a.g.val[j]); \
+        }                                                                                   \
+    }
+    JET_GROUP_LOOP(G, count, APPLY_BODY)
+#undef APPLY_BODY
+    c1 = group_sum<W>(c1, 32);
+    if ((threadIdx.x & 31) == 0 && c1) atomic_add(&a.dev->cut1, c1);
+    if (HIST) {
+        __syncthreads();
+        for (int p = threadIdx.x; p < a.k; p += blockDim.x) if (hs[p]) atomic_add(&a.sizes[p], hs[p]);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.dev->large = large;
+}
+template <class O, class E, class W>
+__device__ __forceinline__ void d_apply_moves(const RefArgs<O, E, W>& a, int group) {
+    switch (group) {
+        case 4: d_apply_moves<4, false, O, E, W>(a, nullptr); break;
+        case 8: d_apply_moves<8, false, O, E, W>(a, nullptr); break;
+        case 16: d_apply_moves<16, false, O, E, W>(a, nullptr); break;
+        default: d_apply_moves<32, false, O, E, W>(a, nullptr); break;
+    }
+}
+// (nclear > 0 and a rebalancing iteration: the bucket totals are zeroed for the
+// next one; their last readers are done)
+template <int G, class O, class E, class W>
+__global__ void __launch_bounds__(BLOCK) k_apply_moves(RefArgs<O, E, W> a, int hist, W* buckets, int64_t nclear, const int* mode) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    if (mode && *mode != 0)
+        for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < nclear; x += (int64_t)gridDim.x * blockDim.x) buckets[x] = 0;
+    if (hist) d_apply_moves<G, true, O, E, W>(a, (W*)smem_raw);
+    else d_apply_moves<G, false, O, E, W>(a, nullptr);
+}
+
+// The first phase for moved rows above HUB_DEG: one block per row.
+template <class O, class E, class W>
+__device__ __forceinline__ void d_apply_hub(const RefArgs<O, E, W>& a) {
+    const O count = a.dev->nmoves_hub;
+    const bool large = a.dev->large != 0;
     for (O x = blockIdx.x; x < count; x += gridDim.x) {
-        O i = a.moves_hub[x];
+        const O i = a.moves_hub[x];
+        const part_t p = a.dest[i];  // the part it left
         const E re = a.g.row[i + 1];
-        for (E j0 = a.g.row[i] + threadIdx.x; j0 < re; j0 += 4 * (E)blockDim.x) {
-            O v[4];
-            uint8_t mk[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = j0 + (E)u * blockDim.x < re ? a.g.adj[j0 + (E)u * blockDim.x] : (O)-1;
-#pragma unroll
-            for (int u = 0; u < 4; u++) mk[u] = v[u] >= 0 ? a.mark[v[u]] : (uint8_t)1;
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-                if (!mk[u]) a.mark[v[u]] = 1;
-        }
+        E j = a.g.row[i] + threadIdx.x;
+        if (large) mark_edges<O, E, W>(a, j, re, (E)blockDim.x);
+        else for (; j < re; j += blockDim.x) conn_sub<O, E, W>(a, a.g.adj[j], p, a.g.val[j]);
     }
 }
 template <class O, class E, class W>
-__global__ void __launch_bounds__(1024) k_mark_neighbors_hub(RefArgs<O, E, W> a) { d_mark_neighbors_hub<O, E, W>(a); }
+__global__ void __launch_bounds__(1024) k_apply_hub(RefArgs<O, E, W> a) { d_apply_hub<O, E, W>(a); }
 
-// perform_moves part 2 (src/jet_refiner.hpp:937-946): cut change from the
-// updated tables.
+// Second phase: edges j0, j0 + stride, ... of a vertex moved from `from` to
+// `to`. Returns the edges' share of the cut change: where the neighbour moved
+// too, what the move changed in the connection to its new part less that to
+// its old one.
+template <class O, class E, class W>
+__device__ __forceinline__ W add_edges(const RefArgs<O, E, W>& a, part_t from, part_t to, uint32_t now, E j0, E re, E stride) {
+    W c = 0;
+    for (E j = j0; j < re; j += stride) {
+        const O v = a.g.adj[j];
+        const W w = a.g.val[j];
+        const bool moved = a.stamp[v] == now;
+        conn_add<O, E, W>(a, v, to, w);
+        if (moved) {
+            const part_t pv = a.part[v], ov = a.dest[v];
+            c += w * (W)((pv == to) - (ov == to) - (pv == from) + (ov == from));
+        }
+    }
+    return c;
+}
+template <int G, class O, class E, class W>
+__device__ __forceinline__ void d_update_add(const RefArgs<O, E, W>& a) {
+    const O count = a.dev->nmoves;
+    const uint32_t now = a.dev->iter + 1;
+    W c2 = 0;
+#define ADD_BODY(x, in, lane)                                                               \
+    {                                                                                       \
+        if (in) {                                                                           \
+            const O i = a.moves[x];                                                         \
+            const E s = a.g.row[i], e = a.g.row[i + 1];                                     \
+            if (e - s <= HUB_DEG) c2 += add_edges<O, E, W>(a, a.dest[i], a.part[i], now, s + lane, e, (E)G); \
+        }                                                                                   \
+    }
+    JET_GROUP_LOOP(G, count, ADD_BODY)
+#undef ADD_BODY
+    c2 = group_sum<W>(c2, 32);
+    if ((threadIdx.x & 31) == 0 && c2) atomic_add(&a.dev->cut2, c2);
+}
+template <class O, class E, class W>
+__device__ __forceinline__ void d_update_add(const RefArgs<O, E, W>& a, int group) {
+    switch (group) {
+        case 4: d_update_add<4, O, E, W>(a); break;
+        case 8: d_update_add<8, O, E, W>(a); break;
+        case 16: d_update_add<16, O, E, W>(a); break;
+        default: d_update_add<32, O, E, W>(a); break;
+    }
+}
+template <class O, class E, class W>
+__device__ __forceinline__ void d_update_add_hub(const RefArgs<O, E, W>& a) {
+    const O count = a.dev->nmoves_hub;
+    const uint32_t now = a.dev->iter + 1;
+    W c2 = 0;
+    for (O x = blockIdx.x; x < count; x += gridDim.x) {
+        const O i = a.moves_hub[x];
+        c2 += add_edges<O, E, W>(a, a.dest[i], a.part[i], now, a.g.row[i] + threadIdx.x, a.g.row[i + 1], (E)blockDim.x);
+    }
+    c2 = group_sum<W>(c2, 32);
+    if ((threadIdx.x & 31) == 0 && c2) atomic_add(&a.dev->cut2, c2);
+}
+
+// After update_large the cut change comes from the rebuilt tables
+// (src/jet_refiner.hpp:937-946): a walk over the moved rows' edges would cost
+// more there than two lookups per move.
 template <class O, class E, class W>
 __device__ __forceinline__ void d_cut_after(RefArgs<O, E, W> a) {
     O count = a.dev->nmoves;
@@ -2276,8 +2338,20 @@ __device__ __forceinline__ void d_cut_after(RefArgs<O, E, W> a) {
     c2 = group_sum<W>(c2, 32);
     if ((threadIdx.x & 31) == 0 && c2) atomic_add(&a.dev->cut2, c2);
 }
-template <class O, class E, class W>
-__global__ void __launch_bounds__(BLOCK) k_cut_after(RefArgs<O, E, W> a) { d_cut_after<O, E, W>(a); }
+// The iteration's cut change (the sums may come from other blocks' atomics:
+// read past L1): the moves' gains before, plus what their connections are
+// after, which without update_large is the gains again and the corrections.
+template <class O, class W>
+__device__ __forceinline__ W cut_change(const RefDev<O, W>* d) {
+    const W c1 = ld_cg(&d->cut1), c2 = ld_cg(&d->cut2);
+    return ld_cg(&d->large) ? c1 + c2 : 2 * c1 + c2;
+}
+template <class O, class W>
+__device__ __forceinline__ void next_iteration(RefDev<O, W>* d) {
+    d->ncand = 0; d->nmoves = 0; d->ncand_hub = 0; d->nmoves_hub = 0; d->nredraw = 0;
+    d->cut1 = 0; d->cut2 = 0; d->large = 0;
+    d->iter++;
+}
 
 // Largest part, results to the host mirror, counters reset.
 template <class O, class E, class W>
@@ -2292,12 +2366,11 @@ __global__ void __launch_bounds__(1024) k_finalize(RefArgs<O, E, W> a, IterResul
         for (int w = 1; w < (int)(blockDim.x >> 5); w++) if (sm[w] > mx) mx = sm[w];
         RefDev<O, W>* d = a.dev;
         out->nmoves = (int64_t)d->nmoves;
-        out->cut_change = (int64_t)(d->cut1 + d->cut2);
+        out->cut_change = (int64_t)cut_change(d);
         out->max_part = (int64_t)mx;
         out->err = d->err;
         out->large = d->large;
-        d->ncand = 0; d->nmoves = 0; d->ncand_hub = 0; d->nmoves_hub = 0; d->nredraw = 0;
-        d->cut1 = 0; d->cut2 = 0; d->large = 0;
+        next_iteration(d);
     }
 }
 
@@ -2363,19 +2436,12 @@ __device__ __forceinline__ void ctl_begin_logic(Ctl<W>* c) {
     c->copy = 0;
     ctl_next_mode(c);
 }
-template <class W>
-__global__ void k_ctl_begin(Ctl<W>* c, CtlHandles h) {
-    ctl_begin_logic(c);
-    ctl_set_handles(c, h, true);
-}
-
 // After an iteration: applies the cut change and largest part, keeps the best
 // state (src/jet_refiner.hpp:1120-1132), evaluates the loop condition and the
 // next mode, and resets the per-iteration counters.
 template <class O, class W>
 __device__ __forceinline__ void ctl_end_logic(Ctl<W>* c, RefDev<O, W>* d, W mx) {
-    // the cut changes were summed by other blocks' atomics: read past L1
-    c->curr_cut -= ld_cg(&d->cut1) + ld_cg(&d->cut2);
+    c->curr_cut -= cut_change(d);
     c->curr_imb = mx > c->opt ? mx - c->opt : 0;
     c->copy = 0;
     if (c->best_imb > c->imb_max && c->curr_imb < c->best_imb) {
@@ -2401,8 +2467,7 @@ __device__ __forceinline__ void ctl_end_logic(Ctl<W>* c, RefDev<O, W>* d, W mx) 
     }
     c->more = more;
     if (more) ctl_next_mode(c);
-    d->ncand = 0; d->nmoves = 0; d->ncand_hub = 0; d->nmoves_hub = 0; d->nredraw = 0;
-    d->cut1 = 0; d->cut2 = 0; d->large = 0;
+    next_iteration(d);
 }
 
 // Largest part size, reduced over the block (result valid in thread 0).
@@ -2420,37 +2485,82 @@ __device__ __forceinline__ W block_max_sizes(const W* sizes, int k) {
     return mx;
 }
 
-// Closes an iteration inside the level graph and sets the graph's handles.
+// What a rebalancing iteration needs to know about the parts, made by the
+// block that closes the iteration before it (or begins the loop).
 template <class O, class E, class W>
-__global__ void __launch_bounds__(1024) k_finalize_ctl(RefArgs<O, E, W> a, Ctl<W>* c, CtlHandles h) {
-    W mx = block_max_sizes<W>(a.sizes, a.k);
-    if (threadIdx.x != 0) return;
-    ctl_end_logic<O, W>(c, a.dev, mx);
-    ctl_set_handles(c, h, true);
+__device__ __forceinline__ void next_prep(const RefArgs<O, E, W>& a, const RebArgs<O, W>& rbw, const RebArgs<O, W>& rbs, int mode) {
+    if (mode == MODE_WEAK) d_weak_prep<O, E, W>(a, rbw);
+    else if (mode == MODE_STRONG) d_strong_prep<O, E, W>(a, rbs);
+}
+template <class O, class E, class W>
+__global__ void __launch_bounds__(1024) k_ctl_begin(RefArgs<O, E, W> a, Ctl<W>* c, CtlHandles h, RebArgs<O, W> rbw, RebArgs<O, W> rbs) {
+    __shared__ int s_mode;
+    if (threadIdx.x == 0) {
+        ctl_begin_logic(c);
+        ctl_set_handles(c, h, true);
+        s_mode = c->mode;
+    }
+    __syncthreads();
+    next_prep<O, E, W>(a, rbw, rbs, s_mode);
 }
 
-// k_cut_after and k_finalize_ctl in one launch (one graph node less per
-// iteration): every block adds its cut change, and the last block to finish
-// (a counter, reset by that block) closes the iteration.
-template <class O, class E, class W>
-__global__ void __launch_bounds__(BLOCK) k_cut_finalize_ctl(RefArgs<O, E, W> a, Ctl<W>* c, CtlHandles h, unsigned* done) {
+// Whether the calling block is the last of the grid to get here (a counter,
+// reset by that block); the other blocks' writes are then visible to it.
+__device__ __forceinline__ bool last_block(unsigned* done) {
     __shared__ int s_last;
-    d_cut_after<O, E, W>(a);
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         s_last = atomicAdd(done, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (!s_last) return;
+    if (!s_last) return false;
     __threadfence();
-    W mx = block_max_sizes<W>(a.sizes, a.k);
-    if (threadIdx.x != 0) return;
-    *done = 0;
-    ctl_end_logic<O, W>(c, a.dev, mx);
-    ctl_set_handles(c, h, true);
+    if (threadIdx.x == 0) *done = 0;
+    return true;
 }
 
+// Closes an iteration inside the level graph: control, handles, and the next
+// rebalance's preparation.
+template <class W, class O>
+struct CloseArgs {
+    Ctl<W>* c;  // null: the iteration is closed by the host loop or a later kernel
+    CtlHandles h;
+    unsigned* done;
+    RebArgs<O, W> rbw, rbs;
+};
+template <class O, class E, class W>
+__device__ __forceinline__ void graph_close(const RefArgs<O, E, W>& a, const CloseArgs<W, O>& cl) {
+    __shared__ int s_mode;
+    W mx = block_max_sizes<W>(a.sizes, a.k);
+    if (threadIdx.x == 0) {
+        ctl_end_logic<O, W>(cl.c, a.dev, mx);
+        ctl_set_handles(cl.c, cl.h, true);
+        s_mode = cl.c->more ? cl.c->mode : MODE_LP;
+    }
+    __syncthreads();
+    next_prep<O, E, W>(a, cl.rbw, cl.rbs, s_mode);
+}
+// The second phase of the moves; the last block closes the iteration.
+template <int G, class O, class E, class W>
+__global__ void __launch_bounds__(BLOCK) k_update_add(RefArgs<O, E, W> a, CloseArgs<W, O> cl) {
+    if (a.dev->large) return;
+    d_update_add<G, O, E, W>(a);
+    if (cl.c && last_block(cl.done)) graph_close<O, E, W>(a, cl);
+}
+template <class O, class E, class W>
+__global__ void __launch_bounds__(1024) k_update_add_hub(RefArgs<O, E, W> a, CloseArgs<W, O> cl) {
+    if (a.dev->large) return;
+    d_update_add_hub<O, E, W>(a);
+    if (cl.c && last_block(cl.done)) graph_close<O, E, W>(a, cl);
+}
+// After update_large: the cut change from the rebuilt tables, and the close.
+template <class O, class E, class W>
+__global__ void __launch_bounds__(BLOCK) k_cut_large(RefArgs<O, E, W> a, CloseArgs<W, O> cl) {
+    if (!a.dev->large) return;
+    d_cut_after<O, E, W>(a);
+    if (cl.c && last_block(cl.done)) graph_close<O, E, W>(a, cl);
+}
 
 // ---------------------------------------------------------------- statistics
 // Cut counted from both endpoints (src/part_stat.hpp:77-108).

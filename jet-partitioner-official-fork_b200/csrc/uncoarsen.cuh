@@ -47,7 +47,8 @@ struct Refiner {
     DBuf<unsigned> lctr;
     // rows of 9-16 and of 17-32 edges (per level) and their counts
     DBuf<O> s16, s32, scnt;
-    DBuf<unsigned> cdone;  // k_cut_finalize_ctl's block counter
+    DBuf<unsigned> cdone;  // block counter of the kernels that close an iteration
+    DBuf<uint32_t> stamp;
     O n_lorder = 0;
     mutable int long_grid_cache = -1;
     // 1: the total edge weight of the finest level is below 2^31, so every
@@ -71,6 +72,7 @@ struct Refiner {
         slots.alloc(slots_cap, s);
         csize.alloc(n1, s); dest_cache.alloc(n1, s); part_work.alloc(n1, s); dest.alloc(n1, s);
         lock.alloc(n1, s); mark.alloc(n1, s); mark.zero();
+        stamp.alloc(n1, s); stamp.zero();
         save_gain.alloc(n1, s); pregain.alloc(n1, s); score.alloc(n1, s);
         cand.alloc(n1, s); cand_hub.alloc(n1, s); moves.alloc(n1, s); moves_hub.alloc(n1, s); bid.alloc(n1, s);
         sizes_curr.alloc(k, s); sizes_best.alloc(k, s); undersized.alloc(k, s); evict_adjust.alloc(k, s);
@@ -132,7 +134,7 @@ struct Refiner {
         RefArgs<O, E, W> a;
         a.g = L.view(); a.k = k; a.coff = coff.p; a.slots = slots.p; a.csize = csize.p; a.dest_cache = dest_cache.p;
         a.lock = lock.p; a.mark = mark.p; a.part = part_work.p; a.dest = dest.p; a.save_gain = save_gain.p;
-        a.pregain = pregain.p; a.sizes = sizes_curr.p; a.cand = cand.p; a.cand_hub = cand_hub.p; a.moves = moves.p;
+        a.pregain = pregain.p; a.stamp = stamp.p; a.sizes = sizes_curr.p; a.cand = cand.p; a.cand_hub = cand_hub.p; a.moves = moves.p;
         a.moves_hub = moves_hub.p; a.dev = dev.p; a.filter = &ctl.p->filter;
         a.narrow = narrow_state > 0 ? 1 : 0;
         a.tw = table_width(L);
@@ -287,9 +289,8 @@ struct Refiner {
 
     // Profiling-pass handles of the current iteration's class brackets.
     int ph[PK_COUNT];
-    int ph_mark = -1;
     DBuf<ProfCounts> pcount;
-    void ph_reset() { for (int i = 0; i < PK_COUNT; i++) ph[i] = -1; ph_mark = -1; phq[0] = phq[1] = -1; }
+    void ph_reset() { for (int i = 0; i < PK_COUNT; i++) ph[i] = -1; phq[0] = phq[1] = -1; }
 
     void lp(const Level<O, E, W>& L) {
         auto a = args(L);
@@ -365,7 +366,7 @@ struct Refiner {
     void weak_select(const Level<O, E, W>& L, RebArgs<O, W>& rb) {
         auto a = args(L);
         int h = ph[PK_REB_SELECT] = prof_begin(s);
-        k_weak_prep<O, E, W><<<1, 1024, 0, s>>>(a, rb); count_launch();
+        if (!capturing()) { k_weak_prep<O, E, W><<<1, 1024, 0, s>>>(a, rb); count_launch(); }
         k_weak_select_thread<O, E, W><<<grid_persistent(L.n, 16), BLOCK, 0, s>>>(a, rb); count_launch();
         if (L.n_warp > 0) { k_weak_select_warp<O, E, W><<<grid_persistent((int64_t)L.n_warp * 32, 16), BLOCK, 0, s>>>(a, rb, L.warp_list.p, L.n_warp); count_launch(); }
         if (L.n_hub > 0) { k_weak_select_warp<O, E, W><<<grid_persistent((int64_t)L.n_hub * 32, 16), BLOCK, 0, s>>>(a, rb, L.hub_list.p, L.n_hub); count_launch(); }
@@ -401,7 +402,7 @@ struct Refiner {
     void strong_select(const Level<O, E, W>& L, RebArgs<O, W>& rb) {
         auto a = args(L);
         int h = ph[PK_REB_SELECT] = prof_begin(s);
-        k_strong_prep<O, E, W><<<1, 1024, 0, s>>>(a, rb); count_launch();
+        if (!capturing()) { k_strong_prep<O, E, W><<<1, 1024, 0, s>>>(a, rb); count_launch(); }
         k_strong_score_thread<O, E, W><<<grid_persistent(L.n, 16), BLOCK, 0, s>>>(a, rb); count_launch();
         if (L.n_warp > 0) { k_strong_score_warp<O, E, W><<<grid_persistent((int64_t)L.n_warp * 32, 16), BLOCK, 0, s>>>(a, rb, L.warp_list.p, L.n_warp); count_launch(); }
         if (L.n_hub > 0) { k_strong_score_warp<O, E, W><<<grid_persistent((int64_t)L.n_hub * 32, 16), BLOCK, 0, s>>>(a, rb, L.hub_list.p, L.n_hub); count_launch(); }
@@ -419,6 +420,7 @@ struct Refiner {
         k_cookie<O, E, W><<<1, 1024, 0, s>>>(a, rb); count_launch();
         k_strong_first<O, E, W><<<grid_persistent(L.n, 8), BLOCK, 0, s>>>(a, rb); count_launch();
         k_strong_redraw<O, E, W><<<1, 1024, 0, s>>>(a, rb); count_launch();
+        k_strong_gain<O, E, W><<<grid_persistent(L.n, 8), BLOCK, 0, s>>>(a); count_launch();
         JET_LAUNCH_CHECK();
         prof_end(h, PK_REB_EVICT, 0, s);
     }
@@ -464,79 +466,65 @@ struct Refiner {
     int64_t q_last = 0;
     int q_fb_last = 0;
 
-    // perform_moves, src/jet_refiner.hpp:905-955, in four parts: the moves
-    // themselves (apply_moves_kernel, which also decides update_small versus
-    // update_large), the small update (subtract pass over all moved vertices,
-    // hubs included, then the add pass), the large update (mark the
-    // neighbours, rebuild their tables) and the cut change.  Both updates'
-    // kernels test the device-side decision, so running both is correct.
-    void apply_moves_kernel(const Level<O, E, W>& L) {
+    // perform_moves, src/jet_refiner.hpp:905-955: the two phases of the moves
+    // (the first decides update_small versus update_large), the rebuild that
+    // update_large needs and its cut change. Every kernel tests the decision
+    // on the device, so running them all is correct. In a level graph (`rb`,
+    // `mode`, `cl`) the first also clears the bucket totals after a rebalance
+    // and the last one that has work closes the iteration.
+    void apply_kernels(const Level<O, E, W>& L, const RebArgs<O, W>* rb = nullptr, const int* mode = nullptr) {
         auto a = args(L);
-        int hist = (size_t)k * sizeof(W) <= 32 * 1024;
-        k_apply_moves<O, E, W><<<grid_persistent(L.n, 8), BLOCK, hist ? (size_t)k * sizeof(W) : 0, s>>>(a, hist); count_launch();
-        JET_LAUNCH_CHECK();
-    }
-    void small_update_kernels(const Level<O, E, W>& L) {
-        auto a = args(L);
-        unsigned grid = grid_persistent((int64_t)L.n * L.group / 4 + 1, 16);
-        const unsigned hub_grid = device_info().sms * 2;
-        // every subtraction before any addition (src/jet_refiner.hpp:786, :810)
+        const unsigned grid = grid_persistent((int64_t)L.n * L.group / 4 + 1, 16);
+        const int hist = (size_t)k * sizeof(W) <= 32 * 1024;
+        const size_t sm = hist ? (size_t)k * sizeof(W) : 0;
+        W* bk = rb ? rb->buckets : nullptr;
+        const int64_t nc = rb ? (int64_t)rb->t_minibuckets + 1 + rb->width : 0;
         switch (L.group) {
-            case 4: k_update_small<4, false, O, E, W><<<grid, BLOCK, 0, s>>>(a); break;
-            case 8: k_update_small<8, false, O, E, W><<<grid, BLOCK, 0, s>>>(a); break;
-            case 16: k_update_small<16, false, O, E, W><<<grid, BLOCK, 0, s>>>(a); break;
-            default: k_update_small<32, false, O, E, W><<<grid, BLOCK, 0, s>>>(a); break;
+            case 4: k_apply_moves<4, O, E, W><<<grid, BLOCK, sm, s>>>(a, hist, bk, nc, mode); break;
+            case 8: k_apply_moves<8, O, E, W><<<grid, BLOCK, sm, s>>>(a, hist, bk, nc, mode); break;
+            case 16: k_apply_moves<16, O, E, W><<<grid, BLOCK, sm, s>>>(a, hist, bk, nc, mode); break;
+            default: k_apply_moves<32, O, E, W><<<grid, BLOCK, sm, s>>>(a, hist, bk, nc, mode); break;
         }
         count_launch();
-        if (L.n_hub > 0) { k_update_small_hub<false, O, E, W><<<hub_grid, 1024, 0, s>>>(a); count_launch(); }
-        switch (L.group) {
-            case 4: k_update_small<4, true, O, E, W><<<grid, BLOCK, 0, s>>>(a); break;
-            case 8: k_update_small<8, true, O, E, W><<<grid, BLOCK, 0, s>>>(a); break;
-            case 16: k_update_small<16, true, O, E, W><<<grid, BLOCK, 0, s>>>(a); break;
-            default: k_update_small<32, true, O, E, W><<<grid, BLOCK, 0, s>>>(a); break;
-        }
-        count_launch();
-        if (L.n_hub > 0) { k_update_small_hub<true, O, E, W><<<hub_grid, 1024, 0, s>>>(a); count_launch(); }
+        if (L.n_hub > 0) { k_apply_hub<O, E, W><<<device_info().sms * 2, 1024, 0, s>>>(a); count_launch(); }
         JET_LAUNCH_CHECK();
     }
-    void large_update_kernels(const Level<O, E, W>& L) {
+    void add_kernels(const Level<O, E, W>& L, const CloseArgs<W, O>& cl) {
         auto a = args(L);
-        unsigned grid = grid_persistent((int64_t)L.n * L.group / 4 + 1, 16);
+        const unsigned grid = grid_persistent((int64_t)L.n * L.group / 4 + 1, 16);
+        CloseArgs<W, O> first = cl;
+        if (L.n_hub > 0) first.c = nullptr;  // the hub kernel closes
         switch (L.group) {
-            case 4: k_mark_neighbors<4, O, E, W><<<grid, BLOCK, 0, s>>>(a); break;
-            case 8: k_mark_neighbors<8, O, E, W><<<grid, BLOCK, 0, s>>>(a); break;
-            case 16: k_mark_neighbors<16, O, E, W><<<grid, BLOCK, 0, s>>>(a); break;
-            default: k_mark_neighbors<32, O, E, W><<<grid, BLOCK, 0, s>>>(a); break;
+            case 4: k_update_add<4, O, E, W><<<grid, BLOCK, 0, s>>>(a, first); break;
+            case 8: k_update_add<8, O, E, W><<<grid, BLOCK, 0, s>>>(a, first); break;
+            case 16: k_update_add<16, O, E, W><<<grid, BLOCK, 0, s>>>(a, first); break;
+            default: k_update_add<32, O, E, W><<<grid, BLOCK, 0, s>>>(a, first); break;
         }
         count_launch();
-        if (L.n_hub > 0) { k_mark_neighbors_hub<O, E, W><<<device_info().sms * 2, 1024, 0, s>>>(a); count_launch(); }
+        if (L.n_hub > 0) { k_update_add_hub<O, E, W><<<device_info().sms * 2, 1024, 0, s>>>(a, cl); count_launch(); }
         JET_LAUNCH_CHECK();
-        if (ph_mark >= 0) {
-            // profiling pass: count the marked rows between the two brackets
-            prof_end(ph_mark, PK_UPDATE_LARGE, 0, s);
-            k_prof_marked<O, E, W><<<grid_persistent(L.n, 4), BLOCK, 0, s>>>(a, pcount.p); count_launch();
-            JET_LAUNCH_CHECK();
-            ph[PK_UPDATE_LARGE] = prof_begin(s);
-        }
-        build_tables(L, 1, &dev.p->large);
     }
-    void cut_after_kernel(const Level<O, E, W>& L) {
-        k_cut_after<O, E, W><<<grid_persistent(L.n, 8), BLOCK, 0, s>>>(args(L)); count_launch();
+    void cut_large_kernel(const Level<O, E, W>& L, const CloseArgs<W, O>& cl) {
+        k_cut_large<O, E, W><<<grid_persistent(L.n, 8), BLOCK, 0, s>>>(args(L), cl); count_launch();
         JET_LAUNCH_CHECK();
     }
     void moves_kernels(const Level<O, E, W>& L) {
-        ph[PK_UPDATE_LARGE] = -1;
+        CloseArgs<W, O> none = {};
         int h = ph[PK_APPLY] = prof_begin(s);
-        apply_moves_kernel(L);
+        apply_kernels(L);
         prof_end(h, PK_APPLY, 0, s);
+        if (h >= 0) {
+            k_prof_marked<O, E, W><<<grid_persistent(L.n, 4), BLOCK, 0, s>>>(args(L), pcount.p); count_launch();
+            JET_LAUNCH_CHECK();
+        }
         h = ph[PK_UPDATE] = prof_begin(s);
-        small_update_kernels(L);
+        add_kernels(L, none);
         prof_end(h, PK_UPDATE, 0, s);
-        ph_mark = prof_begin(s);
-        large_update_kernels(L);
-        if (ph[PK_UPDATE_LARGE] >= 0) prof_end(ph[PK_UPDATE_LARGE], PK_UPDATE_LARGE, 0, s);
+        h = ph[PK_UPDATE_LARGE] = prof_begin(s);
+        build_tables(L, 1, &dev.p->large);
+        prof_end(h, PK_UPDATE_LARGE, 0, s);
         h = ph[PK_CUT_AFTER] = prof_begin(s);
-        cut_after_kernel(L);
+        cut_large_kernel(L, none);
         prof_end(h, PK_CUT_AFTER, 0, s);
     }
 
@@ -590,23 +578,24 @@ struct Refiner {
                 prof_add_bytes(ph[PK_REB_EVICT], evict_full);
             }
         }
-        // apply: per move its vertex, part, destination and weight, the part
-        // and destination writes, the two size updates
-        prof_add_bytes(ph[PK_APPLY], T * (so + 4 + 4 + sw + 4 + 4 + 4) + 2.0 * k * sw);
+        // first phase: per move its vertex, row, part, destination, gain and
+        // weight, the part, destination, cache and stamp writes, the two size
+        // updates; per edge the neighbour's mark (update_large), else the
+        // weight, the neighbour's table offset and size and one slot
+        // read-modify-write
+        const double tbl = so + sw + se + 4 + 2 * sl;
+        prof_add_bytes(ph[PK_APPLY], T * (so + 2 * se + 8 + 2 * sw + 16) + 2.0 * k * sw + Td * (r.large ? so + 1 : tbl));
         if (r.large) {
-            // mark: each moved vertex's row and its neighbours' marks
-            prof_add_bytes(ph_mark, Td * (so + 1) + T * 2 * se);
-            // rebuild: each marked row, its neighbours' parts and the table
+            // rebuild: each marked row, its neighbours' parts and the table;
+            // cut change: per move two lookups in its own table
             prof_add_bytes(ph[PK_UPDATE_LARGE], (double)c.marked * (2 * se + 1 + 4) +
                                                     (double)c.marked_deg * (so + sw + 4) + (double)c.marked_cap * sl);
+            prof_add_bytes(ph[PK_CUT_AFTER], T * (so + se + 4 + 8 + 2 * sl));
         } else {
-            // small update, subtract then add: per moved edge the neighbour,
-            // weight, the neighbour's table offset, size and one slot
-            // read-modify-write, twice
-            prof_add_bytes(ph[PK_UPDATE], 2.0 * Td * (so + sw + se + 4 + 2 * sl) + T * (so + 2 * se + 8));
+            // second phase: per move its row, part and destination; per edge
+            // what the first phase touches, the stamp and the cache
+            prof_add_bytes(ph[PK_UPDATE], T * (so + 2 * se + 8) + Td * (tbl + 8));
         }
-        // cut change part 2: per move two lookups in its own table
-        prof_add_bytes(ph[PK_CUT_AFTER], T * (so + se + 4 + 8 + 2 * sl));
     }
 
     // Host-driven iteration end: results to pinned memory, one host sync.
@@ -815,7 +804,7 @@ struct Refiner {
     void run_level_cta(const Level<O, E, W>& L, part_t* best_part, const Prob& pb, const std::vector<double>& temps, double tol) {
         ctl_init(pb, temps, tol);
         LevelLists<O> li{L.warp_list.p, L.n_warp, L.hub_list.p, L.n_hub, L.group};
-        RebArgs<O, W> rbw = reb_args(L, weak_max_dest(pb.size_max), pb.opt, pb.size_max, false);
+        RebArgs<O, W> rbw = reb_args(L, weak_max_dest(pb.size_max), pb.opt, pb.size_max);
         RebArgs<O, W> rbs = reb_args(L, strong_max_dest(pb.opt, pb.size_max), pb.opt, pb.size_max, false);
         int P = 1;
         while (P < (int)L.n) P <<= 1;
@@ -961,7 +950,7 @@ struct Refiner {
         JET_CUDA(cudaMemsetAsync(cbar.p, 0, sizeof(GridBar), s));
         ctl_init(pb, temps, tol);
         LevelLists<O> li{L.warp_list.p, L.n_warp, L.hub_list.p, L.n_hub, L.group};
-        RebArgs<O, W> rbw = reb_args(L, weak_max_dest(pb.size_max), pb.opt, pb.size_max, false);
+        RebArgs<O, W> rbw = reb_args(L, weak_max_dest(pb.size_max), pb.opt, pb.size_max);
         RebArgs<O, W> rbs = reb_args(L, strong_max_dest(pb.opt, pb.size_max), pb.opt, pb.size_max, false);
         CoopScratch<O, E, W> cs{cbar.p, cwsum.p, chist.p, sk0.p, sk1.p, sv0.p, sv1.p, wpre.p, cmarked.p, coop_qcap(),
                                 coop_boff_cap(), (int64_t)coop_boff_off()};
@@ -1065,7 +1054,7 @@ struct Refiner {
             // the rebalance bodies end in an IF node holding the full sort,
             // which k_reb_ordered opens when the queue cannot be used
             // (a handle must belong to a node: made only where the IF exists)
-            RebArgs<O, W> rbw = reb_args(L, weak_max_dest(pb.size_max), pb.opt, pb.size_max, false);
+            RebArgs<O, W> rbw = reb_args(L, weak_max_dest(pb.size_max), pb.opt, pb.size_max);
             RebArgs<O, W> rbs = reb_args(L, strong_max_dest(pb.opt, pb.size_max), pb.opt, pb.size_max, false);
             cudaGraphConditionalHandle fbw = 0, fbs = 0;
             if (rbw.queue) JET_CUDA(cudaGraphConditionalHandleCreate(&fbw, G, 0, cudaGraphCondAssignDefault));
@@ -1073,14 +1062,17 @@ struct Refiner {
             JET_CUDA(cudaMemsetAsync(dev.p->reb_fb_count, 0, 2 * sizeof(int), s));
             int64_t kb = 0, klp = 0, kw = 0, ks = 0, km = 0, kfw = 0, kfs = 0;
             Ctl<W>* cp = ctl.p;
-            auto t0 = capture_into(G, {}, [&] { k_ctl_begin<W><<<1, 1, 0, s>>>(cp, h); count_launch(); JET_LAUNCH_CHECK(); }, &kb);
+            auto t0 = capture_into(G, {}, [&] {
+                k_ctl_begin<O, E, W><<<1, 1024, 0, s>>>(args(L), cp, h, rbw, rbs); count_launch();
+                JET_LAUNCH_CHECK();
+            }, &kb);
+            const CloseArgs<W, O> cl{cp, h, cdone.p, rbw, rbs};
             cudaGraph_t body, b_lp, b_weak, b_strong, b_copy, b_fbw, b_fbs;
             add_conditional(G, t0, h.loop, cudaGraphCondTypeWhile, &body);
             cudaGraphNode_t n_lp = add_conditional(body, {}, h.lp, cudaGraphCondTypeIf, &b_lp);
             capture_into(b_lp, {}, [&] { lp(L); }, &klp);
             cudaGraphNode_t n_weak = add_conditional(body, {n_lp}, h.weak, cudaGraphCondTypeIf, &b_weak);
             auto tw = capture_into(b_weak, {}, [&] {
-                rbw = reb_args(L, weak_max_dest(pb.size_max), pb.opt, pb.size_max);
                 weak_select(L, rbw);
                 if (rbw.queue) reb_queue<false>(L, rbw, fbw, true);
                 else weak_full(L, rbw);
@@ -1091,7 +1083,6 @@ struct Refiner {
             }
             cudaGraphNode_t n_strong = add_conditional(body, {n_weak}, h.strong, cudaGraphCondTypeIf, &b_strong);
             auto ts = capture_into(b_strong, {}, [&] {
-                rbs = reb_args(L, strong_max_dest(pb.opt, pb.size_max), pb.opt, pb.size_max);
                 strong_select(L, rbs);
                 if (rbs.queue) reb_queue<true>(L, rbs, fbs, true);
                 else strong_full(L, rbs);
@@ -1104,13 +1095,10 @@ struct Refiner {
             // device-side decision: conditional nodes around them cost more
             // than the kernels that return at once)
             auto tm = capture_into(body, {n_strong}, [&] {
-                apply_moves_kernel(L);
-                int hp = prof_begin(s);
-                small_update_kernels(L);
-                large_update_kernels(L);
-                prof_end(hp, PK_UPDATE, 0, s);
-                k_cut_finalize_ctl<O, E, W><<<grid_persistent(L.n, 8), BLOCK, 0, s>>>(args(L), cp, h, cdone.p); count_launch();
-                JET_LAUNCH_CHECK();
+                apply_kernels(L, &rbw, &cp->mode);
+                add_kernels(L, cl);
+                build_tables(L, 1, &dev.p->large);
+                cut_large_kernel(L, cl);
             }, &km);
             add_conditional(body, tm, h.copy, cudaGraphCondTypeIf, &b_copy);
             int64_t kc = 0;

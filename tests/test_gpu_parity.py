@@ -226,6 +226,26 @@ def _skewed_runs(jet, orc, g, og, k, imb, skew, iters_list=(1, 2, 3, 6, 10)):
     return seen
 
 
+@pytest.mark.parametrize("nx,ny,k", [(33, 1, 2), (43, 3, 4), (64, 64, 3), (1621, 1500, 5)],
+                         ids=["one_over_a_warp", "one_over_a_stretch", "whole_stretches", "two_rounds"])
+def test_vertex_pass_edges(jet, graphs, orc, nx, ny, k):
+    """The grid kernels give each warp a stretch of at most 128 vertices:
+    sizes around a warp and a stretch, and one above what the whole grid
+    covers in a round (18,944 warps), in iterations that rebalance and then
+    run LP; parts, moves and cut equal the oracle's."""
+    g = graphs.grid2d(nx, ny, weighted=True, seed=2)
+    og = orc.G.from_csr(g)
+    part = (np.arange(g.n) * k // g.n).astype(np.int32)
+    part[np.random.default_rng(4).random(g.n) < 0.05] = 0
+    for iters in (1, 4):
+        want = orc.refine_iters(og, part, k, 1.03, 0.75, iters)
+        got = jet.refine_iters(g.to("cuda"), torch.from_numpy(part).cuda(), k, 1.03, 0.75, iters)
+        assert got["kinds"] == list(want["kinds"])
+        assert got["moves"] == list(want["moves"])
+        assert np.array_equal(host(got["part"]), want["part"])
+        assert got["cut"] == want["cut"]
+
+
 @pytest.mark.parametrize("n", [8192, 8194, 8450, 130001], ids=["whole_steps", "one_over", "one_step_over", "two_or_more_chunks"])
 @pytest.mark.parametrize("tier", TIERS)
 def test_contract_dense_rows(jet, graphs, orc, tier, n):
