@@ -201,7 +201,7 @@ struct CoopScratch {
 };
 
 // Rebalance tail over the grid (sort_candidates + k_evict_sorted [+ strong]).
-template <bool CL, bool STRONG, class O, class E, class W>
+template <bool CL, bool PASS, bool STRONG, class O, class E, class W>
 __device__ __forceinline__ bool coop_reb_tail(RefArgs<O, E, W>& a, RebArgs<O, W>& rb, CoopScratch<O, E, W>& cs, int bits,
                                               PhaseClock& pc) {
     int* err = &a.dev->err;
@@ -224,7 +224,9 @@ __device__ __forceinline__ bool coop_reb_tail(RefArgs<O, E, W>& a, RebArgs<O, W>
     if (rb.queue) {
         // the grid classifies; block 0 orders the queue (when it fits) and
         // finishes the rebalance while the other blocks wait at the barrier
-        d_reb_classify<STRONG, O, E, W>(a, rb, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+        const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+        if (PASS) d_reb_classify_pass<STRONG, O, E, W>(a, rb, t0, nt);
+        else d_reb_classify<STRONG, O, E, W>(a, rb, t0, nt);
         if (!level_sync<CL>(cs.bar, err)) return false;
         pc.mark(PH_REB_SORT);
         volatile RefDev<O, W>* vd = a.dev;
@@ -294,11 +296,15 @@ __device__ __forceinline__ void coop_zero(W* p, int64_t m) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) p[i] = 0;
 }
 
-template <bool CL, class O, class E, class W>
+// PASS: several vertices per thread, so the passes over all of them take the
+// form that overlaps them (WarpPass).
+template <bool CL, bool PASS, class O, class E, class W>
 __global__ void __launch_bounds__(CTA_THREADS, 1)
 k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, W> rbs, Ctl<W>* c, part_t* best_part,
              W* sizes_best, CoopScratch<O, E, W> cs, int bits, int max_iters) {
     int* err = &a.dev->err;
+    static_assert(REDRAW_CAP * sizeof(O) >= (CTA_THREADS / 32) * PASS_LIST, "the passes' lists share the replay's memory");
+    uint8_t* const pass_list = PASS ? (uint8_t*)redraw_list<O>() : nullptr;
     const O n = a.g.n;
     __shared__ int s_mode;  // of the next iteration, in the block that prepares it
     if (blockIdx.x == 0) {
@@ -316,7 +322,8 @@ k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O,
         const int mode = ((volatile Ctl<W>*)c)->mode;
         if (!more) break;
         if (mode == MODE_LP) {
-            d_lp_select_thread<O, E, W>(a);
+            if (PASS) d_lp_select_pass<O, E, W>(a, pass_list);
+            else d_lp_select_thread<O, E, W>(a);
             d_lp_select_warp<O, E, W>(a, li.warp_list, li.n_warp);
             d_lp_select_warp<O, E, W>(a, li.hub_list, li.n_hub);
             if (!level_sync<CL>(cs.bar, err)) return;
@@ -337,18 +344,20 @@ k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O,
         } else {
             RebArgs<O, W>& rb = mode == MODE_WEAK ? rbw : rbs;
             if (mode == MODE_WEAK) {
-                d_weak_select_thread<O, E, W>(a, rb);
+                if (PASS) d_weak_select_pass<O, E, W>(a, rb, pass_list);
+                else d_weak_select_thread<O, E, W>(a, rb);
                 d_weak_select_warp<O, E, W>(a, rb, li.warp_list, li.n_warp);
                 d_weak_select_warp<O, E, W>(a, rb, li.hub_list, li.n_hub);
             } else {
-                d_strong_score_thread<O, E, W>(a, rb);
+                if (PASS) d_strong_score_pass<O, E, W>(a, rb, pass_list);
+                else d_strong_score_thread<O, E, W>(a, rb);
                 d_strong_score_warp<O, E, W>(a, rb, li.warp_list, li.n_warp);
                 d_strong_score_warp<O, E, W>(a, rb, li.hub_list, li.n_hub);
             }
             if (!level_sync<CL>(cs.bar, err)) return;
             pc.mark(PH_REB_SELECT);
-            bool ok = mode == MODE_WEAK ? coop_reb_tail<CL, false, O, E, W>(a, rb, cs, bits, pc)
-                                        : coop_reb_tail<CL, true, O, E, W>(a, rb, cs, bits, pc);
+            bool ok = mode == MODE_WEAK ? coop_reb_tail<CL, PASS, false, O, E, W>(a, rb, cs, bits, pc)
+                                        : coop_reb_tail<CL, PASS, true, O, E, W>(a, rb, cs, bits, pc);
             if (!ok) return;
         }
         // perform_moves (src/jet_refiner.hpp:905-955)

@@ -1646,6 +1646,13 @@ __global__ void k_strong_first(RefArgs<O, E, W> a, RebArgs<O, W> rb) { d_strong_
 
 // One block: sorts the queued vertices by id and replays their draws in order.
 static constexpr int REDRAW_CAP = 4096;
+// (the persistent grid keeps the vertex passes' lists here too: a barrier
+// lies between the two uses)
+template <class O>
+__device__ __forceinline__ O* redraw_list() {
+    __shared__ O list[REDRAW_CAP];
+    return list;
+}
 template <class K>
 __device__ __forceinline__ void block_sort_keys(K* key, int P) {
     for (int k = 2; k <= P; k <<= 1) {
@@ -1704,7 +1711,7 @@ static constexpr int REDRAW_ES_CAP = 513;
 template <class O, class E, class W>
 __device__ __forceinline__ void d_strong_redraw(RefArgs<O, E, W> a, RebArgs<O, W> rb, unsigned char* stage = nullptr,
                                                 size_t stage_bytes = 0) {
-    __shared__ O list[REDRAW_CAP];
+    O* const list = redraw_list<O>();
     __shared__ W es_s[REDRAW_ES_CAP];
     O cnt = a.dev->nredraw;
     if (cnt == 0) return;

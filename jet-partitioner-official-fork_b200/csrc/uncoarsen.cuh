@@ -762,13 +762,17 @@ struct Refiner {
         return (v && *v) ? std::atoll(v) : def;
     }
     static int64_t cta_prefer_n() { static const int64_t v = bound("JET_CTA_PREFER_N", CTA_PREFER_N); return v; }
-    static int64_t cluster_max_n() {
+    int64_t cluster_max_n() const {
         // batch and server workers share the GPU: their bound is separate
-        static const int64_t v = bound("JET_CLUSTER_MAX_N", CLUSTER_MAX_N);
+        static const int64_t v = bound("JET_CLUSTER_MAX_N", 0);
         static const int64_t vb = bound("JET_BATCH_CLUSTER_MAX_N", CLUSTER_MAX_N);
-        return batch_thread() ? vb : v;
+        if (batch_thread()) return vb;
+        return v > 0 ? v : (k <= MANY_PARTS ? CLUSTER_MAX_N : CLUSTER_MAX_N_MANY);
     }
-    static int64_t coop_max_n() { static const int64_t v = bound("JET_COOP_MAX_N", COOP_MAX_N); return v; }
+    int64_t coop_max_n() const {
+        static const int64_t v = bound("JET_COOP_MAX_N", 0);
+        return v > 0 ? v : (k <= MANY_PARTS ? COOP_MAX_N : COOP_MAX_N_MANY);
+    }
     static int64_t cluster_max_m() { static const int64_t v = bound("JET_PERSISTENT_MAX_M", CLUSTER_MAX_M); return v; }
     static int64_t coop_max_m() { static const int64_t v = bound("JET_PERSISTENT_MAX_M", COOP_MAX_M); return v; }
     bool cta_eligible(const Level<O, E, W>& L) const {
@@ -825,10 +829,16 @@ struct Refiner {
     }
 
     // ------------------------------------------------------------ cooperative loop
-    // Above these the multi-kernel graph is faster (128^3 mesh: the 241,769-
-    // vertex level, 3.1 M entries, runs 86 against 111 us per iteration here;
-    // the 749,582-vertex level gains nothing and the 2 M one loses).
-    static constexpr int64_t COOP_MAX_N = (int64_t)1 << 18;
+    // Above these the multi-kernel graph is as fast or faster. us per iteration
+    // in the graph and here: 2D mesh of 1 M vertices into 64 parts 88 and 55,
+    // geometric graph of 800,000 (8 M entries) into 32 92 and 61, 128^3 mesh's
+    // 749,582-vertex level (7.5 M) into 64 103 and 88, 100^3 mesh into 256 103 and
+    // 90, a 504,000-vertex mesh into 300 104 and 78; but 128^3's finest level (2.1 M,
+    // 12.5 M entries) 107 and 110-116. With many parts a rebalance queues more
+    // candidates than the grid's block orders (COOP_QUEUE_KEYS) and takes the
+    // full sort: 717,120 vertices into 768 parts 111 and 146 (387,988: 114 and 107).
+    static constexpr int64_t COOP_MAX_N = (int64_t)1 << 20;
+    static constexpr int64_t COOP_MAX_N_MANY = (int64_t)1 << 18;
     // Parts up to which the persistent loops take a level whose rows fit the
     // warps' shared-memory tables. 717k-vertex mesh into 768 parts: its levels
     // of 1,323-61,159 vertices ran 98-297 us per iteration as level graphs
@@ -836,7 +846,7 @@ struct Refiner {
     // which Metis 73); beyond about 1,000 parts the bucket arrays (50 per part
     // and section) outgrow the blocks' shared memory and the gain.
     static constexpr part_t LEVEL_MAX_K = 1024;
-    static constexpr int64_t COOP_MAX_M = (int64_t)1 << 22;
+    static constexpr int64_t COOP_MAX_M = (int64_t)1 << 23;
     size_t coop_smem(const Level<O, E, W>& L) const {
         size_t kw = (size_t)table_width(L);
         size_t nw = CTA_THREADS / 32;
@@ -872,7 +882,7 @@ struct Refiner {
     size_t coop_static_smem() const {
         static size_t bytes = [] {
             cudaFuncAttributes fa;
-            return cudaFuncGetAttributes(&fa, k_level_coop<false, O, E, W>) == cudaSuccess ? fa.sharedSizeBytes : (size_t)1 << 30;
+            return cudaFuncGetAttributes(&fa, k_level_coop<false, false, O, E, W>) == cudaSuccess ? fa.sharedSizeBytes : (size_t)1 << 30;
         }();
         return bytes;
     }
@@ -887,6 +897,12 @@ struct Refiner {
     // 260 vs 131 us per iteration at 242k mesh vertices; 2x slower on dense
     // power-law levels of tens of millions of entries.
     static constexpr int64_t CLUSTER_MAX_N = (int64_t)1 << 16;
+    // (more parts than this: every block reads and scans 50 bucket totals per
+    // part, which 16 blocks do no faster than 148; 768 parts, 33,618 vertices 117
+    // us per iteration in the cluster and 107 in the grid, 61,251 vertices 133 and
+    // 109. 32 parts, 65,536 vertices: 36 and 41)
+    static constexpr part_t MANY_PARTS = 512;
+    static constexpr int64_t CLUSTER_MAX_N_MANY = (int64_t)1 << 15;
     static constexpr int64_t CLUSTER_MAX_M = (int64_t)1 << 21;
     // CTAs in the level cluster: 16 where the device allows it, else 8, 0 if
     // no cluster of 1024-thread CTAs with this shared memory fits.
@@ -897,7 +913,7 @@ struct Refiner {
         if (cluster_cache >= 0 && cluster_cache_smem == smem) return cluster_cache;
         cluster_cache_smem = smem;
         cluster_cache = [smem] {
-            const void* f = (const void*)k_level_coop<true, O, E, W>;
+            const void* f = (const void*)k_level_coop<true, false, O, E, W>;
             if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem(f)) != cudaSuccess) return 0;
             cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             for (int want : {16, 8}) {
@@ -932,14 +948,18 @@ struct Refiner {
     void run_level_coop(const Level<O, E, W>& L, part_t* best_part, const Prob& pb, const std::vector<double>& temps, double tol,
                         bool cluster = false) {
         size_t smem = coop_smem(L);
+        // two vertices per thread and more: the overlapping passes (at 1.6 the
+        // plain ones were 1-2 us a phase faster)
+        const bool pass = (int64_t)L.n > 2 * (int64_t)CTA_THREADS * device_info().sms;
+        const void* const grid_kernel =
+            pass ? (const void*)k_level_coop<false, true, O, E, W> : (const void*)k_level_coop<false, false, O, E, W>;
         int grid = 0;
         if (cluster) {
             grid = cluster_size(L);
         } else {
-            JET_CUDA(cudaFuncSetAttribute(k_level_coop<false, O, E, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          max_dynamic_smem((const void*)k_level_coop<false, O, E, W>)));
+            JET_CUDA(cudaFuncSetAttribute(grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem(grid_kernel)));
             int per_sm = 0;
-            JET_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_level_coop<false, O, E, W>, CTA_THREADS, smem));
+            JET_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grid_kernel, CTA_THREADS, smem));
             if (per_sm < 1) throw JetError{JET_ERR_CUDA, "cooperative level kernel does not fit on an SM"};
             grid = device_info().sms * per_sm;
         }
@@ -973,10 +993,10 @@ struct Refiner {
             at.val.clusterDim.z = 1;
             cfg.attrs = &at;
             cfg.numAttrs = 1;
-            JET_CUDA(cudaLaunchKernelEx(&cfg, k_level_coop<true, O, E, W>, a, li, rbw, rbs, cp, bp, sb, cs, bits, max_iters));
+            JET_CUDA(cudaLaunchKernelEx(&cfg, k_level_coop<true, false, O, E, W>, a, li, rbw, rbs, cp, bp, sb, cs, bits, max_iters));
         } else {
             void* params[] = {&a, &li, &rbw, &rbs, &cp, &bp, &sb, &cs, &bits, &max_iters};
-            JET_CUDA(cudaLaunchCooperativeKernel((const void*)k_level_coop<false, O, E, W>, dim3(grid), dim3(CTA_THREADS), params, smem, s));
+            JET_CUDA(cudaLaunchCooperativeKernel(grid_kernel, dim3(grid), dim3(CTA_THREADS), params, smem, s));
         }
         count_launch();
         ctl_finish();
