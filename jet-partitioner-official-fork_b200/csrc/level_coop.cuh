@@ -304,6 +304,7 @@ k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O,
              W* sizes_best, CoopScratch<O, E, W> cs, int bits, int max_iters) {
     int* err = &a.dev->err;
     static_assert(REDRAW_CAP * sizeof(O) >= (CTA_THREADS / 32) * PASS_LIST, "the passes' lists share the replay's memory");
+    static_assert(REDRAW_CAP * sizeof(O) >= CTA_THREADS * sizeof(W), "so do the afterburner's sums");
     uint8_t* const pass_list = PASS ? (uint8_t*)redraw_list<O>() : nullptr;
     const O n = a.g.n;
     __shared__ int s_mode;  // of the next iteration, in the block that prepares it
@@ -328,12 +329,7 @@ k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O,
             d_lp_select_warp<O, E, W>(a, li.hub_list, li.n_hub);
             if (!level_sync<CL>(cs.bar, err)) return;
             pc.mark(PH_LP_SELECT);
-            switch (li.group) {
-                case 4: d_afterburn<4, O, E, W>(a); break;
-                case 8: d_afterburn<8, O, E, W>(a); break;
-                case 16: d_afterburn<16, O, E, W>(a); break;
-                default: d_afterburn<32, O, E, W>(a); break;
-            }
+            d_afterburn_walk<O, E, W>(a, (W*)redraw_list<O>());
             if (!level_sync<CL>(cs.bar, err)) return;
             pc.mark(PH_AFTERBURN);
             if (li.n_hub > 0) {
@@ -361,7 +357,7 @@ k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O,
             if (!ok) return;
         }
         // perform_moves (src/jet_refiner.hpp:905-955)
-        d_apply_moves<O, E, W>(a, li.group);
+        d_apply_walk<O, E, W>(a);
         if (mode != MODE_LP)  // for the next rebalance: the last one is done with them
             coop_zero<O, E, W>(rbw.buckets, (int64_t)rbw.t_minibuckets + 1 + rbw.width);
         if (!level_sync<CL>(cs.bar, err)) return;
@@ -372,7 +368,7 @@ k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O,
             pc.mark(PH_UPDATE_SUB);
         }
         if (!ld_cg(&a.dev->large)) {
-            d_update_add<O, E, W>(a, li.group);
+            d_add_walk<O, E, W>(a);
             if (li.n_hub > 0) d_update_add_hub<O, E, W>(a);
         } else {
             // update_large: queue the marked rows (one coalesced pass), then

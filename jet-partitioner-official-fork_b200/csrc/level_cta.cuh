@@ -24,7 +24,6 @@ struct LevelLists {
     O n_warp;
     const O* hub_list;
     O n_hub;
-    int group;
 };
 
 // Exclusive scan of in[0..n) into out (may alias), over the block: each
@@ -278,12 +277,7 @@ k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, 
             d_lp_select_warp<O, E, W>(a, li.hub_list, li.n_hub);
             __syncthreads();
             pc.mark(PH_LP_SELECT);
-            switch (li.group) {
-                case 4: d_afterburn<4, O, E, W>(a); break;
-                case 8: d_afterburn<8, O, E, W>(a); break;
-                case 16: d_afterburn<16, O, E, W>(a); break;
-                default: d_afterburn<32, O, E, W>(a); break;
-            }
+            d_afterburn_walk<O, E, W>(a, (W*)redraw_list<O>());
             __syncthreads();
             pc.mark(PH_AFTERBURN);
             d_afterburn_hub<O, E, W>(a);
@@ -305,7 +299,7 @@ k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, 
             d_reb_tail<true, O, E, W>(a, rbs, keys, P, pc);
         }
         // perform_moves (src/jet_refiner.hpp:905-955)
-        d_apply_moves<O, E, W>(a, li.group);
+        d_apply_walk<O, E, W>(a);
         if (mode != MODE_LP) cta_zero_buckets<O, E, W>(rbw);  // for the next rebalance: the last one is done with them
         __syncthreads();
         pc.mark(PH_APPLY);
@@ -315,7 +309,7 @@ k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, 
             pc.mark(PH_UPDATE_SUB);
         }
         if (!a.dev->large) {
-            d_update_add<O, E, W>(a, li.group);
+            d_add_walk<O, E, W>(a);
             if (li.n_hub > 0) d_update_add_hub<O, E, W>(a);
             __syncthreads();
             pc.mark(PH_UPDATE_ADD);

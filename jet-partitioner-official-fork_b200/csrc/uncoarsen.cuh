@@ -807,7 +807,7 @@ struct Refiner {
 
     void run_level_cta(const Level<O, E, W>& L, part_t* best_part, const Prob& pb, const std::vector<double>& temps, double tol) {
         ctl_init(pb, temps, tol);
-        LevelLists<O> li{L.warp_list.p, L.n_warp, L.hub_list.p, L.n_hub, L.group};
+        LevelLists<O> li{L.warp_list.p, L.n_warp, L.hub_list.p, L.n_hub};
         RebArgs<O, W> rbw = reb_args(L, weak_max_dest(pb.size_max), pb.opt, pb.size_max);
         RebArgs<O, W> rbs = reb_args(L, strong_max_dest(pb.opt, pb.size_max), pb.opt, pb.size_max, false);
         int P = 1;
@@ -969,7 +969,7 @@ struct Refiner {
         if (cmarked.n < (int64_t)n_max) cmarked.alloc(n_max > 0 ? n_max : 1, s);
         JET_CUDA(cudaMemsetAsync(cbar.p, 0, sizeof(GridBar), s));
         ctl_init(pb, temps, tol);
-        LevelLists<O> li{L.warp_list.p, L.n_warp, L.hub_list.p, L.n_hub, L.group};
+        LevelLists<O> li{L.warp_list.p, L.n_warp, L.hub_list.p, L.n_hub};
         RebArgs<O, W> rbw = reb_args(L, weak_max_dest(pb.size_max), pb.opt, pb.size_max);
         RebArgs<O, W> rbs = reb_args(L, strong_max_dest(pb.opt, pb.size_max), pb.opt, pb.size_max, false);
         CoopScratch<O, E, W> cs{cbar.p, cwsum.p, chist.p, sk0.p, sk1.p, sv0.p, sv1.p, wpre.p, cmarked.p, coop_qcap(),

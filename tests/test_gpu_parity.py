@@ -265,6 +265,20 @@ def test_contract_dense_rows(jet, graphs, orc, tier, n):
     assert np.array_equal(host(got.val), want.val) and np.array_equal(host(got.vw), want.vw)
 
 
+def test_moves_walk_many(jet, graphs, orc):
+    """More moves than 32 for every warp of the grid (18,944 warps): the walk
+    over the moved rows takes more than one round. A random partition of a
+    2.4 M-vertex mesh, one iteration; parts, moves and cut equal the oracle's."""
+    g = graphs.grid2d(1621, 1500, weighted=True, seed=2)
+    part = np.random.default_rng(4).integers(0, 5, g.n).astype(np.int32)
+    want = orc.refine_iters(orc.G.from_csr(g), part, 5, 1.10, 0.75, 1)
+    got = jet.refine_iters(g.to("cuda"), torch.from_numpy(part).cuda(), 5, 1.10, 0.75, 1)
+    assert want["moves"][0] > 32 * 18944
+    assert got["moves"] == list(want["moves"])
+    assert np.array_equal(host(got["part"]), want["part"])
+    assert got["cut"] == want["cut"]
+
+
 @pytest.mark.parametrize("tier", ["i32", "big"])
 def test_rebalance_queue_overflow_falls_back(jet, graphs, orc, tier):
     """A 250 x 250 mesh with 90% of its vertices piled into one part: the
