@@ -2229,8 +2229,9 @@ __global__ void __launch_bounds__(1024) k_reb_ordered(RefArgs<O, E, W> a, RebArg
 // second phase meets on its way (stamp). Before, the moves, the two table
 // passes and the lookups after them were four phases with a barrier or a
 // launch each. Per iteration, before and after (128^3 mesh into 64 parts, levels
-// of 3,971 / 70,288 / 749,582 / 2.1 M vertices): 64 / 70 / 112 / 118 us, now
+// of 3,971 / 70,288 / 749,582 / 2.1 M vertices): 64 / 70 / 112 / 118 us and
 // 55 / 57 / 103 / 107; a 65,536-vertex 2D mesh level in the cluster 44 -> 36.
+// (The walk of the persistent loops, warp_rows, then took the first two to 48 / 52.)
 // update_small subtract (src/jet_refiner.hpp:786-808).
 template <class O, class E, class W>
 __device__ __forceinline__ void conn_sub(const RefArgs<O, E, W>& a, O v, part_t p, W w) {
