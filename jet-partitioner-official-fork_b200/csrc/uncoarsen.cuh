@@ -761,17 +761,19 @@ struct Refiner {
         const char* v = std::getenv(env);
         return (v && *v) ? std::atoll(v) : def;
     }
+    // Every value counts as set: 0 leaves no level to a driver.
+    static constexpr int64_t UNSET = std::numeric_limits<int64_t>::min();
     static int64_t cta_prefer_n() { static const int64_t v = bound("JET_CTA_PREFER_N", CTA_PREFER_N); return v; }
     int64_t cluster_max_n() const {
         // batch and server workers share the GPU: their bound is separate
-        static const int64_t v = bound("JET_CLUSTER_MAX_N", 0);
+        static const int64_t v = bound("JET_CLUSTER_MAX_N", UNSET);
         static const int64_t vb = bound("JET_BATCH_CLUSTER_MAX_N", CLUSTER_MAX_N);
         if (batch_thread()) return vb;
-        return v > 0 ? v : (k <= MANY_PARTS ? CLUSTER_MAX_N : CLUSTER_MAX_N_MANY);
+        return v != UNSET ? v : (k <= MANY_PARTS ? CLUSTER_MAX_N : CLUSTER_MAX_N_MANY);
     }
     int64_t coop_max_n() const {
-        static const int64_t v = bound("JET_COOP_MAX_N", 0);
-        return v > 0 ? v : (k <= MANY_PARTS ? COOP_MAX_N : COOP_MAX_N_MANY);
+        static const int64_t v = bound("JET_COOP_MAX_N", UNSET);
+        return v != UNSET ? v : (k <= MANY_PARTS ? COOP_MAX_N : COOP_MAX_N_MANY);
     }
     static int64_t cluster_max_m() { static const int64_t v = bound("JET_PERSISTENT_MAX_M", CLUSTER_MAX_M); return v; }
     static int64_t coop_max_m() { static const int64_t v = bound("JET_PERSISTENT_MAX_M", COOP_MAX_M); return v; }
