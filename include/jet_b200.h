@@ -294,7 +294,10 @@ int64_t jet_launch_count(void);
  *     JET_ERR_TIMEOUT when a wait ran out; *passed = barrier passages.
  *   jet_test_table_overflow: inserts parts 0..nparts-1 into a shared-memory
  *     connectivity table of `cap` slots (k parts) with the table-build insert;
- *     JET_ERR_OVERFLOW when the probe bound flagged a full table. */
+ *     JET_ERR_OVERFLOW when the probe bound flagged a full table.
+ *   jet_test_bucket_copy: bucket offsets that each block of a cluster or grid
+ *     loop keeps in shared memory for a level of n vertices, all or none,
+ *     within `budget` bytes; < 0: -(error code). Host arithmetic only. */
 int jet_test_inject_metis_failures(int count);
 /* Coarsest-graph Metis calls of this process: out[6] = {calls served by helper
  * processes, helper calls whose transfer failed (rerun in-process, the helper
@@ -304,6 +307,7 @@ int jet_test_inject_metis_failures(int count);
 int jet_metis_call_stats(int64_t* out);
 int jet_test_grid_barrier(int blocks, int absent_block, int spin_cap_log2, int rounds, int* passed);
 int jet_test_table_overflow(int cap, int k, int nparts, int* claimed);
+int64_t jet_test_bucket_copy(int tier, int64_t n, int32_t k, int64_t budget);
 
 /* Device memory for callers without a CUDA toolchain of their own (the C++
  * drop-in include/jet.h uses these for the device views it allocates, as

@@ -1,5 +1,6 @@
 // test_hooks.cu -- entry points that let tests drive the library's failure
-// handling without faulting, trapping or hanging a GPU.  No counterpart in
+// handling without faulting, trapping or hanging a GPU, and see a decision
+// that no result shows.  No counterpart in
 // the reference, which has no failure handling to test (a Metis failure
 // exits the process, src/initial_partition.hpp:106-109).
 //
@@ -15,6 +16,9 @@
 //                           parts than slots the probe bound must flag
 //                           ERRF_OVERFLOW (JET_ERR_OVERFLOW), writing nothing
 //                           outside the table.
+//   jet_test_bucket_copy    how many bucket offsets each block of a cluster or
+//                           grid loop keeps in shared memory for a level
+//                           (host arithmetic only).
 #include "uncoarsen.cuh"
 #include <string>
 
@@ -73,6 +77,16 @@ extern "C" int jet_test_grid_barrier(int blocks, int absent_block, int spin_cap_
         return JET_ERR_TIMEOUT;
     }
     return JET_OK;
+}
+
+extern "C" int64_t jet_test_bucket_copy(int tier, int64_t n, int32_t k, int64_t budget) {
+    if (n < 1 || k < 1 || budget < 0 || (tier != 2 && n > INT32_MAX)) return -JET_ERR_INVALID;
+    switch (tier) {
+        case 0: return Refiner<int32_t, int32_t, int32_t>::bucket_copy((int32_t)n, k, (size_t)budget);
+        case 1: return Refiner<int32_t, int64_t, int64_t>::bucket_copy((int32_t)n, k, (size_t)budget);
+        case 2: return Refiner<int64_t, int64_t, int64_t>::bucket_copy(n, k, (size_t)budget);
+        default: return -JET_ERR_INVALID;
+    }
 }
 
 extern "C" int jet_test_table_overflow(int cap, int k, int nparts, int* claimed_out) {

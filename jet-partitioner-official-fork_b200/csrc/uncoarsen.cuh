@@ -78,7 +78,7 @@ struct Refiner {
         sizes_curr.alloc(k, s); sizes_best.alloc(k, s); undersized.alloc(k, s); evict_adjust.alloc(k, s);
         evict_start.alloc(k + 1, s);
         O sections, tmb;
-        sections_for(nmax, sections, tmb);
+        sections_for(nmax, k, sections, tmb);
         bucket_cap = (int64_t)tmb + 1 + (int64_t)MAX_BUCKETS * sections;
         buckets.alloc(bucket_cap, s);
         boff.alloc(bucket_cap, s);
@@ -120,7 +120,7 @@ struct Refiner {
     }
 
     // src/jet_refiner.hpp:425-430 and :559-564
-    void sections_for(O n, O& sections, O& t_minibuckets) const {
+    static void sections_for(O n, part_t k, O& sections, O& t_minibuckets) {
         sections = MAX_SECTIONS;
         O section_size = (n + sections * k) / (sections * k);
         if (section_size < 4096) {
@@ -333,7 +333,7 @@ struct Refiner {
     RebArgs<O, W> reb_args(const Level<O, E, W>& L, W max_dest, W opt, W size_max, bool clear = true) {
         RebArgs<O, W> rb;
         O sections, tmb;
-        sections_for(L.n, sections, tmb);
+        sections_for(L.n, k, sections, tmb);
         rb.size_max = size_max; rb.opt = opt; rb.max_dest = max_dest; rb.sections = sections; rb.t_minibuckets = tmb;
         rb.width = MAX_BUCKETS * sections; rb.buckets = buckets.p; rb.boff = boff.p; rb.bid = bid.p; rb.score = score.p;
         rb.undersized = undersized.p; rb.evict_adjust = evict_adjust.p; rb.evict_start = evict_start.p;
@@ -558,7 +558,7 @@ struct Refiner {
             const double evict_full = n * (4 + so + sw + 4) + T * (so + 4);
             if (phq[0] >= 0) {
                 O sections, tmb;
-                sections_for(L.n, sections, tmb);
+                sections_for(L.n, k, sections, tmb);
                 const double nb = (double)tmb + 1, m = (double)q_last, cand = (double)c.reb_cand;
                 // queue path: bucket scan (read, write), every vertex's bucket
                 // id, each candidate's part and weight, the bucket offsets and
@@ -853,7 +853,7 @@ struct Refiner {
         size_t kw = (size_t)table_width(L);
         size_t nw = CTA_THREADS / 32;
         size_t conn = ((nw * kw * sizeof(part_t) + 15) & ~(size_t)15) + nw * kw * sizeof(W);
-        size_t q = (size_t)coop_boff_off() + (size_t)coop_boff_cap() * sizeof(W);
+        size_t q = (size_t)coop_boff_off() + (size_t)coop_boff_cap(L) * sizeof(W);
         return (conn > q ? conn : q) + 64;
     }
     // the per-block bucket offsets sit past both the queue keys and the full
@@ -869,19 +869,25 @@ struct Refiner {
     // the loop's global accesses hit)
     static constexpr int COOP_QUEUE_KEYS = 2048;
     int coop_qcap() const { return COOP_QUEUE_KEYS; }
-    // bucket offsets every block of the persistent grid keeps in shared
-    // memory after the keys: room for the largest level the grid drivers
-    // take, within 160 KiB (else those levels scan them across the grid)
-    int64_t coop_boff_cap() const {
-        int64_t nmax = (int64_t)n_max;
-        const int64_t lim = coop_max_n() > cluster_max_n() ? coop_max_n() : cluster_max_n();
-        if (nmax > lim) nmax = lim;
+    // Bucket offsets that every block of a cluster or grid loop keeps in shared
+    // memory after the keys: all of them for a level of n vertices when they
+    // take at most `budget` bytes, else none (the loop then scans them across
+    // the grid, with a barrier or two more per rebalance).
+    static int64_t bucket_copy(O n, part_t k, size_t budget) {
         O sections, tmb;
-        sections_for((O)nmax, sections, tmb);
+        sections_for(n, k, sections, tmb);
         const int64_t want = (int64_t)tmb + 1;
-        return want * (int64_t)sizeof(W) <= ((int64_t)160 << 10) ? want : 0;
+        return want * (int64_t)sizeof(W) <= (int64_t)budget ? want : 0;
     }
-    size_t coop_static_smem() const {
+    // 160 KiB, or what the kernel's other shared memory leaves of an SM's (64-bit
+    // weights: 150 KiB, 384 parts at one section)
+    static size_t bucket_copy_budget() {
+        const size_t rest = (size_t)coop_boff_off() + coop_static_smem() + 64, all = (size_t)device_info().max_smem_optin;
+        const size_t left = all > rest ? all - rest : 0;
+        return left < ((size_t)160 << 10) ? left : (size_t)160 << 10;
+    }
+    int64_t coop_boff_cap(const Level<O, E, W>& L) const { return bucket_copy(L.n, k, bucket_copy_budget()); }
+    static size_t coop_static_smem() {
         static size_t bytes = [] {
             cudaFuncAttributes fa;
             return cudaFuncGetAttributes(&fa, k_level_coop<false, false, O, E, W>) == cudaSuccess ? fa.sharedSizeBytes : (size_t)1 << 30;
@@ -975,7 +981,7 @@ struct Refiner {
         RebArgs<O, W> rbw = reb_args(L, weak_max_dest(pb.size_max), pb.opt, pb.size_max);
         RebArgs<O, W> rbs = reb_args(L, strong_max_dest(pb.opt, pb.size_max), pb.opt, pb.size_max, false);
         CoopScratch<O, E, W> cs{cbar.p, cwsum.p, chist.p, sk0.p, sk1.p, sv0.p, sv1.p, wpre.p, cmarked.p, coop_qcap(),
-                                coop_boff_cap(), (int64_t)coop_boff_off()};
+                                coop_boff_cap(L), (int64_t)coop_boff_off()};
         int bits = bits_for((uint64_t)rbw.none_key);
         int max_iters = 1 << 22;
         RefArgs<O, E, W> a = args(L);

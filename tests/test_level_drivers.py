@@ -1,5 +1,6 @@
 """Which level loop a level goes to: the bounds between the drivers, and what
 each loop reserves. Results do not depend on it; the parity tests cover those."""
+import ctypes
 import json
 import os
 import subprocess
@@ -44,3 +45,37 @@ def test_a_bound_of_zero_leaves_a_driver_out():
         assert _drivers(JET_CLUSTER_MAX_N=value) == (cut, {"cta", "coop"})
     assert _drivers(JET_COOP_MAX_N="0", JET_CLUSTER_MAX_N="0") == (cut, {"cta"})
     assert _drivers(JET_COOP_MAX_N="1000000") == (cut, {"cta", "cluster", "coop"})
+
+
+# what a cluster's or grid's block has for the bucket offsets: 160 KiB with
+# 32-bit weights, what its other shared memory leaves with 64-bit ones
+@pytest.mark.parametrize("tier,k,budget,n,want", [
+    (0, 64, 160 << 10, 3971, 50 * 64 + 1), (0, 64, 160 << 10, 1 << 20, 50 * 64 * 5 + 1), (0, 256, 160 << 10, 60000, 50 * 256 + 1),
+    (0, 819, 160 << 10, 60000, 50 * 819 + 1), (0, 820, 160 << 10, 60000, 0), (1, 205, 150 << 10, 60000, 50 * 205 + 1),
+    (1, 256, 150 << 10, 1 << 18, 50 * 256 + 1), (1, 256, 150 << 10, 1 << 20, 0), (2, 384, 150 << 10, 60000, 0),
+    (2, 383, 150 << 10, 60000, 50 * 383 + 1)])
+def test_bucket_offsets_reserved_for_the_level(jet, tier, k, budget, n, want):
+    """The reservation follows the level's own size, whatever the largest
+    level that the loop could take."""
+    f = jet.load().jet_test_bucket_copy
+    f.restype = ctypes.c_int64
+    assert f(tier, ctypes.c_int64(n), ctypes.c_int32(k), ctypes.c_int64(budget)) == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tier", ["big", "biggest"])
+@pytest.mark.parametrize("k", [380, 400, 409, 512])
+def test_wide_weights_and_many_parts_keep_the_persistent_loops(jet, graphs, orc, tier, k):
+    """64-bit weights: bucket offsets of 385 to 409 parts fit 160 KiB but not
+    what the kernel's other shared memory leaves; such levels run on the
+    cluster and the grid all the same, with the grid-wide scan."""
+    g = graphs.rgg(90000, 9.0, seed=5).as_tier(tier)
+    g.val = g.val * (2 ** 31 // int(g.val.sum()) + 1)
+    assert int(g.val.sum()) > 2 ** 31
+    want, wcut, _ = orc.partition(orc.G.from_csr(g), k, alg=1, imb=1.05, seed=4)
+    fn = {"big": jet.partition_big, "biggest": jet.partition_biggest}[tier]
+    jet.prof_phases(True)
+    part, cut, _ = fn(jet.config_t(coarsening_alg=1, num_parts=k, max_imb_ratio=1.05), g.to("cuda"), seed=4)
+    ran = {d for d, p in jet.prof_phases(False).items() if p}
+    assert {"cluster", "coop"} <= ran
+    assert cut == wcut and (part.cpu().numpy() == want).all()
