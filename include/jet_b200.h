@@ -297,7 +297,10 @@ int64_t jet_launch_count(void);
  *     JET_ERR_OVERFLOW when the probe bound flagged a full table.
  *   jet_test_bucket_copy: bucket offsets that each block of a cluster or grid
  *     loop keeps in shared memory for a level of n vertices, all or none,
- *     within `budget` bytes; < 0: -(error code). Host arithmetic only. */
+ *     within `budget` bytes; < 0: -(error code). Host arithmetic only.
+ *   jet_test_long_rows: 1 when the persistent loops give each row of a level
+ *     a group of lanes, 0 when they walk the rows as one sequence per warp. Host
+ *     arithmetic only. */
 int jet_test_inject_metis_failures(int count);
 /* Coarsest-graph Metis calls of this process: out[6] = {calls served by helper
  * processes, helper calls whose transfer failed (rerun in-process, the helper
@@ -308,6 +311,7 @@ int jet_metis_call_stats(int64_t* out);
 int jet_test_grid_barrier(int blocks, int absent_block, int spin_cap_log2, int rounds, int* passed);
 int jet_test_table_overflow(int cap, int k, int nparts, int* claimed);
 int64_t jet_test_bucket_copy(int tier, int64_t n, int32_t k, int64_t budget);
+int jet_test_long_rows(int64_t n, int64_t m, int64_t max_deg, int64_t n_hub);
 
 /* Device memory for callers without a CUDA toolchain of their own (the C++
  * drop-in include/jet.h uses these for the device views it allocates, as

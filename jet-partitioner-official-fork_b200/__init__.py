@@ -59,6 +59,7 @@ EXPORTED_SYMBOLS = [
     "jet_server_footprint", "jet_server_stats_get", "jet_server_destroy", "jet_refine_hierarchy",
     "jet_device_alloc", "jet_device_free", "jet_copy", "jet_read_metis", "jet_free_host",
     "jet_test_inject_metis_failures", "jet_test_grid_barrier", "jet_test_table_overflow", "jet_test_bucket_copy",
+    "jet_test_long_rows",
     "jet_prof_phases", "jet_metis_call_stats",
 ]
 

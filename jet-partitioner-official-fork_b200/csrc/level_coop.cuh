@@ -297,8 +297,9 @@ __device__ __forceinline__ void coop_zero(W* p, int64_t m) {
 }
 
 // PASS: several vertices per thread, so the passes over all of them take the
-// form that overlaps them (WarpPass).
-template <bool CL, bool PASS, class O, class E, class W>
+// form that overlaps them (WarpPass). LONG: the level has long rows
+// (Refiner::long_rows).
+template <bool CL, bool PASS, bool LONG, class O, class E, class W>
 __global__ void __launch_bounds__(CTA_THREADS, 1)
 k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, W> rbs, Ctl<W>* c, part_t* best_part,
              W* sizes_best, CoopScratch<O, E, W> cs, int bits, int max_iters) {
@@ -329,7 +330,7 @@ k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O,
             d_lp_select_warp<O, E, W>(a, li.hub_list, li.n_hub);
             if (!level_sync<CL>(cs.bar, err)) return;
             pc.mark(PH_LP_SELECT);
-            d_afterburn_walk<O, E, W>(a, (W*)redraw_list<O>());
+            loop_afterburn<LONG, O, E, W>(a, li.group, (W*)redraw_list<O>());
             if (!level_sync<CL>(cs.bar, err)) return;
             pc.mark(PH_AFTERBURN);
             if (li.n_hub > 0) {
@@ -357,7 +358,7 @@ k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O,
             if (!ok) return;
         }
         // perform_moves (src/jet_refiner.hpp:905-955)
-        d_apply_walk<O, E, W>(a);
+        loop_apply<LONG, O, E, W>(a, li.group);
         if (mode != MODE_LP)  // for the next rebalance: the last one is done with them
             coop_zero<O, E, W>(rbw.buckets, (int64_t)rbw.t_minibuckets + 1 + rbw.width);
         if (!level_sync<CL>(cs.bar, err)) return;
@@ -368,7 +369,7 @@ k_level_coop(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O,
             pc.mark(PH_UPDATE_SUB);
         }
         if (!ld_cg(&a.dev->large)) {
-            d_add_walk<O, E, W>(a);
+            loop_add<LONG, O, E, W>(a, li.group);
             if (li.n_hub > 0) d_update_add_hub<O, E, W>(a);
         } else {
             // update_large: queue the marked rows (one coalesced pass), then

@@ -24,6 +24,7 @@ struct LevelLists {
     O n_warp;
     const O* hub_list;
     O n_hub;
+    int group;  // lanes per row, where rows have a group (Level::group)
 };
 
 // Exclusive scan of in[0..n) into out (may alias), over the block: each
@@ -224,7 +225,8 @@ __device__ __forceinline__ void cta_place(unsigned char* base, uint32_t off, T*&
     ptr = dst;
 }
 
-template <class O, class E, class W>
+// LONG: the level has long rows (Refiner::long_rows).
+template <bool LONG, class O, class E, class W>
 __global__ void __launch_bounds__(CTA_THREADS, 1)
 k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, W> rbs, Ctl<W>* c, part_t* best_part,
             W* sizes_best, int P, int max_iters, CtaSmemPlan plan) {
@@ -277,7 +279,7 @@ k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, 
             d_lp_select_warp<O, E, W>(a, li.hub_list, li.n_hub);
             __syncthreads();
             pc.mark(PH_LP_SELECT);
-            d_afterburn_walk<O, E, W>(a, (W*)redraw_list<O>());
+            loop_afterburn<LONG, O, E, W>(a, li.group, (W*)redraw_list<O>());
             __syncthreads();
             pc.mark(PH_AFTERBURN);
             d_afterburn_hub<O, E, W>(a);
@@ -299,7 +301,7 @@ k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, 
             d_reb_tail<true, O, E, W>(a, rbs, keys, P, pc);
         }
         // perform_moves (src/jet_refiner.hpp:905-955)
-        d_apply_walk<O, E, W>(a);
+        loop_apply<LONG, O, E, W>(a, li.group);
         if (mode != MODE_LP) cta_zero_buckets<O, E, W>(rbw);  // for the next rebalance: the last one is done with them
         __syncthreads();
         pc.mark(PH_APPLY);
@@ -309,7 +311,7 @@ k_level_cta(RefArgs<O, E, W> a, LevelLists<O> li, RebArgs<O, W> rbw, RebArgs<O, 
             pc.mark(PH_UPDATE_SUB);
         }
         if (!a.dev->large) {
-            d_add_walk<O, E, W>(a);
+            loop_add<LONG, O, E, W>(a, li.group);
             if (li.n_hub > 0) d_update_add_hub<O, E, W>(a);
             __syncthreads();
             pc.mark(PH_UPDATE_ADD);

@@ -1056,10 +1056,11 @@ __global__ void __launch_bounds__(BLOCK) k_lp_select_warp(RefArgs<O, E, W> a, co
 // search over the lanes' running degrees. For the persistent level loops: with
 // a fixed group of 4-32 lanes per vertex their few warps took many rounds, and the
 // work per vertex ran on one lane of the group. Whole calls 5-11% faster (2D mesh
-// of 63,511 vertices, ultra settings, 48.3 -> 43.5 ms; 128^3 45.7 -> 43.0 ms). The
-// grid kernels keep the groups: they have warps enough, and a warp that
-// draws several of a power-law graph's long rows holds up the launch (R-MAT 2^24's
-// apply kernels 135 ms in groups, 227 ms as a walk).
+// of 63,511 vertices, ultra settings, 48.3 -> 43.5 ms; 128^3 45.7 -> 43.0 ms). A
+// warp that draws several of a power-law graph's long rows holds up the phase,
+// so levels of long rows keep the groups (Refiner::long_rows), and so do the
+// grid kernels, which have warps enough (R-MAT 2^24's apply kernels 135 ms in
+// groups, 227 ms as a walk).
 // Rows above HUB_DEG are left out (degree 0 here).
 // item(in, i, degree, p, q): sets the two values; called by every lane.
 // edge(j, ok, owner, p, q): U edges (ok: present), their owners' lanes and values.
@@ -2498,6 +2499,49 @@ __device__ __forceinline__ void d_update_add_hub(const RefArgs<O, E, W>& a) {
     }
     c2 = group_sum<W>(c2, 32);
     if ((threadIdx.x & 31) == 0 && c2) atomic_add(&a.dev->cut2, c2);
+}
+
+// The persistent level loops' forms of the afterburner and of the moves' two
+// phases. LONG: a group of lanes per row, as in the grid kernels; else the
+// rows' edges as one sequence per warp.
+template <bool LONG, class O, class E, class W>
+__device__ __forceinline__ void loop_afterburn(const RefArgs<O, E, W>& a, int group, W* sums) {
+    if (!LONG) {
+        d_afterburn_walk<O, E, W>(a, sums);
+        return;
+    }
+    switch (group) {
+        case 4: d_afterburn<4, O, E, W>(a); break;
+        case 8: d_afterburn<8, O, E, W>(a); break;
+        case 16: d_afterburn<16, O, E, W>(a); break;
+        default: d_afterburn<32, O, E, W>(a); break;
+    }
+}
+template <bool LONG, class O, class E, class W>
+__device__ __forceinline__ void loop_apply(const RefArgs<O, E, W>& a, int group) {
+    if (!LONG) {
+        d_apply_walk<O, E, W>(a);
+        return;
+    }
+    switch (group) {
+        case 4: d_apply_moves<4, false, O, E, W>(a, nullptr); break;
+        case 8: d_apply_moves<8, false, O, E, W>(a, nullptr); break;
+        case 16: d_apply_moves<16, false, O, E, W>(a, nullptr); break;
+        default: d_apply_moves<32, false, O, E, W>(a, nullptr); break;
+    }
+}
+template <bool LONG, class O, class E, class W>
+__device__ __forceinline__ void loop_add(const RefArgs<O, E, W>& a, int group) {
+    if (!LONG) {
+        d_add_walk<O, E, W>(a);
+        return;
+    }
+    switch (group) {
+        case 4: d_update_add<4, O, E, W>(a); break;
+        case 8: d_update_add<8, O, E, W>(a); break;
+        case 16: d_update_add<16, O, E, W>(a); break;
+        default: d_update_add<32, O, E, W>(a); break;
+    }
 }
 
 // After update_large the cut change comes from the rebuilt tables

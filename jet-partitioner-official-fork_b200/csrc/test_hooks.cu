@@ -19,6 +19,8 @@
 //   jet_test_bucket_copy    how many bucket offsets each block of a cluster or
 //                           grid loop keeps in shared memory for a level
 //                           (host arithmetic only).
+//   jet_test_long_rows      whether the persistent loops give a level's rows a
+//                           group of lanes each (host arithmetic only).
 #include "uncoarsen.cuh"
 #include <string>
 
@@ -87,6 +89,10 @@ extern "C" int64_t jet_test_bucket_copy(int tier, int64_t n, int32_t k, int64_t 
         case 2: return Refiner<int64_t, int64_t, int64_t>::bucket_copy(n, k, (size_t)budget);
         default: return -JET_ERR_INVALID;
     }
+}
+
+extern "C" int jet_test_long_rows(int64_t n, int64_t m, int64_t max_deg, int64_t n_hub) {
+    return Refiner<int64_t, int64_t, int64_t>::long_rows(n, m, max_deg, n_hub) ? 1 : 0;
 }
 
 extern "C" int jet_test_table_overflow(int cap, int k, int nparts, int* claimed_out) {

@@ -777,6 +777,21 @@ struct Refiner {
     }
     static int64_t cluster_max_m() { static const int64_t v = bound("JET_PERSISTENT_MAX_M", CLUSTER_MAX_M); return v; }
     static int64_t coop_max_m() { static const int64_t v = bound("JET_PERSISTENT_MAX_M", COOP_MAX_M); return v; }
+    // Levels whose rows the persistent loops give a group of lanes each, instead
+    // of walking them as one sequence per warp (warp_rows): rows of very uneven
+    // length, where a warp that draws several long ones holds up the phase (hub
+    // rows, or a mean of 32 edges and a longest row of four times that), and small
+    // dense levels, whose every row fills the warps by itself (a mean of 32 and
+    // of a sixteenth of the vertices). us per iteration as walks and in groups:
+    // R-MAT levels into 32 parts, 26,710 vertices (mean 62) 494 and 301, 8,593
+    // (173) 308 and 222, 480 (209) 101 and 91; the first with 64-bit weights 807
+    // and 527; HEC's R-MAT level of 22,427 (91) 1,296 and 732. Even rows are
+    // better walked: geometric graphs of 15,058 vertices (mean 180) 149 and 159,
+    // 33,258 (42) 108 and 110, 132,498 (13) 45 and 54.
+    static bool long_rows(int64_t n, int64_t m, int64_t max_deg, int64_t n_hub) {
+        return n_hub > 0 || (m >= 32 * n && (max_deg * n >= 4 * m || 16 * m >= n * n));
+    }
+    static bool long_rows(const Level<O, E, W>& L) { return long_rows((int64_t)L.n, (int64_t)L.m, (int64_t)L.max_deg, (int64_t)L.n_hub); }
     bool cta_eligible(const Level<O, E, W>& L) const {
         int64_t cap = (use_cluster && !batch_thread() && cluster_size(L) > 0) ? cta_prefer_n() : CTA_MAX_N;
         return use_cta && (int64_t)L.n <= cap && (int64_t)L.m <= CTA_MAX_M && k <= CTA_MAX_K;
@@ -809,7 +824,7 @@ struct Refiner {
 
     void run_level_cta(const Level<O, E, W>& L, part_t* best_part, const Prob& pb, const std::vector<double>& temps, double tol) {
         ctl_init(pb, temps, tol);
-        LevelLists<O> li{L.warp_list.p, L.n_warp, L.hub_list.p, L.n_hub};
+        LevelLists<O> li{L.warp_list.p, L.n_warp, L.hub_list.p, L.n_hub, L.group};
         RebArgs<O, W> rbw = reb_args(L, weak_max_dest(pb.size_max), pb.opt, pb.size_max);
         RebArgs<O, W> rbs = reb_args(L, strong_max_dest(pb.opt, pb.size_max), pb.opt, pb.size_max, false);
         int P = 1;
@@ -817,14 +832,14 @@ struct Refiner {
         size_t scratch = level_cta_smem<O, W>(P, table_width(L)) + 64;
         // the attribute is per function and process-wide: always the device
         // maximum, so concurrent callers with different sizes cannot race
-        const size_t smax = max_dynamic_smem((const void*)k_level_cta<O, E, W>);
-        JET_CUDA(cudaFuncSetAttribute(k_level_cta<O, E, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax));
+        auto* const kernel = long_rows(L) ? k_level_cta<true, O, E, W> : k_level_cta<false, O, E, W>;
+        const size_t smax = max_dynamic_smem((const void*)kernel);
+        JET_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax));
         // the level's table slots, as init_conn counted them
         const int64_t nslots = last_slots;
         const int64_t nbuckets = (int64_t)rbw.t_minibuckets + 1 + rbw.width;
         CtaSmemPlan plan = plan_cta_smem<O, W>((int64_t)L.n, nslots, nbuckets, k, scratch, smax, cta_smem_resident());
-        k_level_cta<O, E, W><<<1, CTA_THREADS, plan.total, s>>>(args(L), li, rbw, rbs, ctl.p, best_part, sizes_best.p, P,
-                                                                 1 << 22, plan);
+        kernel<<<1, CTA_THREADS, plan.total, s>>>(args(L), li, rbw, rbs, ctl.p, best_part, sizes_best.p, P, 1 << 22, plan);
         count_launch();
         JET_LAUNCH_CHECK();
         ctl_finish();
@@ -889,8 +904,15 @@ struct Refiner {
     int64_t coop_boff_cap(const Level<O, E, W>& L) const { return bucket_copy(L.n, k, bucket_copy_budget()); }
     static size_t coop_static_smem() {
         static size_t bytes = [] {
-            cudaFuncAttributes fa;
-            return cudaFuncGetAttributes(&fa, k_level_coop<false, false, O, E, W>) == cudaSuccess ? fa.sharedSizeBytes : (size_t)1 << 30;
+            size_t most = 0;
+            for (const void* f : {(const void*)k_level_coop<true, false, false, O, E, W>, (const void*)k_level_coop<true, false, true, O, E, W>,
+                                  (const void*)k_level_coop<false, false, false, O, E, W>, (const void*)k_level_coop<false, true, false, O, E, W>,
+                                  (const void*)k_level_coop<false, false, true, O, E, W>}) {
+                cudaFuncAttributes fa;
+                if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) return (size_t)1 << 30;
+                if (fa.sharedSizeBytes > most) most = fa.sharedSizeBytes;
+            }
+            return most;
         }();
         return bytes;
     }
@@ -921,7 +943,7 @@ struct Refiner {
         if (cluster_cache >= 0 && cluster_cache_smem == smem) return cluster_cache;
         cluster_cache_smem = smem;
         cluster_cache = [smem] {
-            const void* f = (const void*)k_level_coop<true, false, O, E, W>;
+            const void* f = (const void*)k_level_coop<true, false, false, O, E, W>;
             if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem(f)) != cudaSuccess) return 0;
             cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             for (int want : {16, 8}) {
@@ -958,9 +980,11 @@ struct Refiner {
         size_t smem = coop_smem(L);
         // two vertices per thread and more: the overlapping passes (at 1.6 the
         // plain ones were 1-2 us a phase faster)
-        const bool pass = (int64_t)L.n > 2 * (int64_t)CTA_THREADS * device_info().sms;
-        const void* const grid_kernel =
-            pass ? (const void*)k_level_coop<false, true, O, E, W> : (const void*)k_level_coop<false, false, O, E, W>;
+        const bool lng = long_rows(L);
+        const bool pass = !lng && (int64_t)L.n > 2 * (int64_t)CTA_THREADS * device_info().sms;
+        const void* const grid_kernel = lng    ? (const void*)k_level_coop<false, false, true, O, E, W>
+                                        : pass ? (const void*)k_level_coop<false, true, false, O, E, W>
+                                               : (const void*)k_level_coop<false, false, false, O, E, W>;
         int grid = 0;
         if (cluster) {
             grid = cluster_size(L);
@@ -977,7 +1001,7 @@ struct Refiner {
         if (cmarked.n < (int64_t)n_max) cmarked.alloc(n_max > 0 ? n_max : 1, s);
         JET_CUDA(cudaMemsetAsync(cbar.p, 0, sizeof(GridBar), s));
         ctl_init(pb, temps, tol);
-        LevelLists<O> li{L.warp_list.p, L.n_warp, L.hub_list.p, L.n_hub};
+        LevelLists<O> li{L.warp_list.p, L.n_warp, L.hub_list.p, L.n_hub, L.group};
         RebArgs<O, W> rbw = reb_args(L, weak_max_dest(pb.size_max), pb.opt, pb.size_max);
         RebArgs<O, W> rbs = reb_args(L, strong_max_dest(pb.opt, pb.size_max), pb.opt, pb.size_max, false);
         CoopScratch<O, E, W> cs{cbar.p, cwsum.p, chist.p, sk0.p, sk1.p, sv0.p, sv1.p, wpre.p, cmarked.p, coop_qcap(),
@@ -1001,7 +1025,10 @@ struct Refiner {
             at.val.clusterDim.z = 1;
             cfg.attrs = &at;
             cfg.numAttrs = 1;
-            JET_CUDA(cudaLaunchKernelEx(&cfg, k_level_coop<true, false, O, E, W>, a, li, rbw, rbs, cp, bp, sb, cs, bits, max_iters));
+            auto* const kernel = lng ? k_level_coop<true, false, true, O, E, W> : k_level_coop<true, false, false, O, E, W>;
+            JET_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem((const void*)kernel)));
+            JET_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            JET_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, li, rbw, rbs, cp, bp, sb, cs, bits, max_iters));
         } else {
             void* params[] = {&a, &li, &rbw, &rbs, &cp, &bp, &sb, &cs, &bits, &max_iters};
             JET_CUDA(cudaLaunchCooperativeKernel(grid_kernel, dim3(grid), dim3(CTA_THREADS), params, smem, s));

@@ -7,6 +7,7 @@ import subprocess
 import sys
 
 import pytest
+import torch
 
 from conftest import ROOT
 
@@ -78,4 +79,67 @@ def test_wide_weights_and_many_parts_keep_the_persistent_loops(jet, graphs, orc,
     part, cut, _ = fn(jet.config_t(coarsening_alg=1, num_parts=k, max_imb_ratio=1.05), g.to("cuda"), seed=4)
     ran = {d for d, p in jet.prof_phases(False).items() if p}
     assert {"cluster", "coop"} <= ran
+    assert cut == wcut and (part.cpu().numpy() == want).all()
+
+
+@pytest.mark.parametrize("n,m,max_deg,n_hub,want", [
+    (10000, 60000, 60, 0, 0), (10000, 60000, 5000, 1, 1),                          # a mesh; one hub row
+    (10000, 320000, 127, 0, 0), (10000, 320000, 128, 0, 1),                        # longest row of four times the mean
+    (10000, 319999, 4000, 0, 0),                                                   # a mean below 32
+    (513, 16416, 60, 0, 0), (512, 16384, 60, 0, 1), (200000, 26000000, 300, 0, 0)  # small and dense; large and dense
+])
+def test_levels_of_long_rows(jet, n, m, max_deg, n_hub, want):
+    """The rule that gives rows groups of lanes, at its edges."""
+    assert jet.load().jet_test_long_rows(*(ctypes.c_int64(x) for x in (n, m, max_deg, n_hub))) == want
+
+
+@pytest.fixture(scope="module")
+def long_row_graphs(graphs, orc):
+    """Graphs with hub rows or long uneven ones, and the oracle's partitions, made once each."""
+    made = {}
+
+    def get(tier, wide, kind, k, alg):
+        key = (tier, wide, kind, k, alg)
+        if key in made:
+            return made[key]
+        if kind == "rmat":
+            g = graphs.rmat(16, 8, seed=4, tier=tier)
+            assert int((g.row[1:] - g.row[:-1]).max()) > 4096
+        elif kind == "star":  # short rows and one hub
+            n = 9000
+            u = torch.cat([torch.zeros(5000, dtype=torch.long), torch.arange(1, n - 1)])
+            v = torch.cat([torch.arange(1, 5001), torch.arange(2, n)])
+            g = graphs.from_undirected(n, u, v, torch.randint(1, 5, (u.numel(),), generator=torch.Generator().manual_seed(1)))
+        else:  # every row a tenth of the vertices, no hub
+            n = 1500
+            a, b = torch.randint(0, n, (2, 110000), generator=torch.Generator().manual_seed(2))
+            pairs = torch.unique((torch.minimum(a, b) * n + torch.maximum(a, b))[a != b])
+            g = graphs.from_undirected(n, pairs // n, pairs % n, pairs % 8 + 1)
+        g = g.as_tier(tier)
+        if wide:
+            g.val = g.val * (2 ** 31 // int(g.val.sum()) + 1)
+        want, cut, _ = orc.partition(orc.G.from_csr(g), k, alg=alg, imb=1.05, seed=3)
+        made[key] = g, want, cut
+        return made[key]
+    return get
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("drivers", ["all", "cta", "cluster", "coop"])
+@pytest.mark.parametrize("tier,wide", [("i32", False), ("big", True), ("biggest", True)])
+@pytest.mark.parametrize("kind,k,alg", [("rmat", 48, 0), ("rmat", 40, 1), ("star", 8, 0), ("dense", 24, 1)])
+def test_long_rows_on_the_persistent_loops(jet, long_row_graphs, drivers, tier, wide, kind, k, alg):
+    """Levels with hub rows and of long uneven rows, in 32 bits and with
+    weight sums above 2^31, on each loop: equal to the oracle."""
+    g, want, wcut = long_row_graphs(tier, wide, kind, k, alg)
+    assert not wide or int(g.val.sum()) > 2 ** 31
+    q = jet.DRIVER_REB_QUEUE
+    mask = {"all": jet.DRIVER_ALL, "cta": jet.DRIVER_CTA | q, "cluster": jet.DRIVER_CLUSTER | q,
+            "coop": jet.DRIVER_COOP | jet.DRIVER_GRAPH | q}[drivers]
+    fn = {"i32": jet.partition, "big": jet.partition_big, "biggest": jet.partition_biggest}[tier]
+    prev = jet.set_refine_drivers(mask)
+    try:
+        part, cut, _ = fn(jet.config_t(coarsening_alg=alg, num_parts=k, max_imb_ratio=1.05), g.to("cuda"), seed=3)
+    finally:
+        jet.set_refine_drivers(prev)
     assert cut == wcut and (part.cpu().numpy() == want).all()
