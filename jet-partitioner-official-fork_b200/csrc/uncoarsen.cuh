@@ -771,12 +771,15 @@ struct Refiner {
         if (batch_thread()) return vb;
         return v != UNSET ? v : (k <= MANY_PARTS ? CLUSTER_MAX_N : CLUSTER_MAX_N_MANY);
     }
-    int64_t coop_max_n() const {
+    int64_t coop_max_n(const Level<O, E, W>& L) const {
         static const int64_t v = bound("JET_COOP_MAX_N", UNSET);
-        return v != UNSET ? v : (k <= MANY_PARTS ? COOP_MAX_N : COOP_MAX_N_MANY);
+        return v != UNSET ? v : (k <= MANY_PARTS && !long_rows(L) ? COOP_MAX_N : COOP_MAX_N_MANY);
     }
     static int64_t cluster_max_m() { static const int64_t v = bound("JET_PERSISTENT_MAX_M", CLUSTER_MAX_M); return v; }
-    static int64_t coop_max_m() { static const int64_t v = bound("JET_PERSISTENT_MAX_M", COOP_MAX_M); return v; }
+    static int64_t coop_max_m(const Level<O, E, W>& L) {
+        static const int64_t v = bound("JET_PERSISTENT_MAX_M", UNSET);
+        return v != UNSET ? v : (sizeof(W) == 8 && long_rows(L) ? COOP_MAX_M_LONG : COOP_MAX_M);
+    }
     // Levels whose rows the persistent loops give a group of lanes each, instead
     // of walking them as one sequence per warp (warp_rows): rows of very uneven
     // length, where a warp that draws several long ones holds up the phase (hub
@@ -854,8 +857,12 @@ struct Refiner {
     // 12.5 M entries) 107 and 110-116. With many parts a rebalance queues more
     // candidates than the grid's block orders (COOP_QUEUE_KEYS) and takes the
     // full sort: 717,120 vertices into 768 parts 111 and 146 (387,988: 114 and 107).
+    // Nor do levels of long rows gain above that bound (R-MAT 2^19 into 64 parts:
+    // finest level 365 and 489), and with 64-bit weights they lose from fewer
+    // entries on (R-MAT 2^19's levels of 6-8 M entries 434-604 in the graph and 590-749).
     static constexpr int64_t COOP_MAX_N = (int64_t)1 << 20;
     static constexpr int64_t COOP_MAX_N_MANY = (int64_t)1 << 18;
+    static constexpr int64_t COOP_MAX_M_LONG = (int64_t)1 << 22;
     // Parts up to which the persistent loops take a level whose rows fit the
     // warps' shared-memory tables. 717k-vertex mesh into 768 parts: its levels
     // of 1,323-61,159 vertices ran 98-297 us per iteration as level graphs
@@ -917,8 +924,8 @@ struct Refiner {
         return bytes;
     }
     bool coop_eligible(const Level<O, E, W>& L) const {
-        return use_coop && device_info().coop && !cta_eligible(L) && (int64_t)L.n <= coop_max_n() &&
-               (int64_t)L.m <= coop_max_m() && k <= LEVEL_MAX_K && table_width(L) <= WARP_TABLE &&
+        return use_coop && device_info().coop && !cta_eligible(L) && (int64_t)L.n <= coop_max_n(L) &&
+               (int64_t)L.m <= coop_max_m(L) && k <= LEVEL_MAX_K && table_width(L) <= WARP_TABLE &&
                coop_smem(L) + coop_static_smem() <= (size_t)device_info().max_smem_optin;
     }
 

@@ -143,3 +143,20 @@ def test_long_rows_on_the_persistent_loops(jet, long_row_graphs, drivers, tier, 
     finally:
         jet.set_refine_drivers(prev)
     assert cut == wcut and (part.cpu().numpy() == want).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale,degree,tier,wide,loops", [
+    (18, 8, "i32", False, {"coop"}), (19, 8, "i32", False, set()), (18, 10, "i32", False, {"coop"}),
+    (18, 8, "big", True, {"coop"}), (18, 10, "big", True, set())])
+def test_large_levels_of_long_rows_stay_level_graphs(jet, graphs, scale, degree, tier, wide, loops):
+    """Power-law levels above 262,144 vertices, and with 64-bit weights above
+    2^22 entries, are faster as level graphs than on the grid."""
+    g = graphs.rmat(scale, degree, seed=4, tier=tier, device="cuda").as_tier(tier)
+    assert (g.nnz > 1 << 22) == (degree == 10 or scale == 19)
+    if wide:
+        g.val = g.val * (2 ** 31 // int(g.val.sum()) + 1)
+    part = torch.randint(0, 16, (g.n,), generator=torch.Generator().manual_seed(1), dtype=torch.int32).cuda()
+    jet.prof_phases(True)
+    jet.refine_level(g, part, 16, 1.10)
+    assert {d for d, p in jet.prof_phases(False).items() if p} == loops
