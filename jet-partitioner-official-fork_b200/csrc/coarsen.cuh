@@ -59,13 +59,14 @@ __device__ __forceinline__ void argmax_merge(W& bw, E& bj, W w2, E j2) {
 // total order, so the edge order does not matter), four edges per round with
 // the neighbour ids, weights and neighbour weights all loaded before the first use.
 template <class O, class E, class W>
-__device__ __forceinline__ void heavy_edges(const GView<O, E, W>& g, W max_allowed, E j0, E e, E stride, W& bw, E& bj) {
+__device__ __forceinline__ void heavy_edges(const GView<O, E, W>& g, W max_allowed, Cursor<E> j0, Cursor<E> e, Cursor<E> stride, W& bw,
+                                            E& bj) {
     for (; j0 < e; j0 += 4 * stride) {
         O v[4];
         W w[4], vw[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            const E j = j0 + (E)u * stride;
+            const Cursor<E> j = j0 + u * stride;
             v[u] = j < e ? g.adj[j] : (O)-1;
             w[u] = j < e ? g.val[j] : (W)0;
         }
@@ -73,7 +74,7 @@ __device__ __forceinline__ void heavy_edges(const GView<O, E, W>& g, W max_allow
         for (int u = 0; u < 4; u++) vw[u] = v[u] >= 0 ? g.vw[v[u]] : max_allowed;
 #pragma unroll
         for (int u = 0; u < 4; u++)
-            if (vw[u] < max_allowed) argmax_merge<O, E, W>(bw, bj, w[u], j0 + (E)u * stride);
+            if (vw[u] < max_allowed) argmax_merge<O, E, W>(bw, bj, w[u], (E)(j0 + u * stride));
     }
 }
 
@@ -87,7 +88,7 @@ __global__ void __launch_bounds__(BLOCK) k_hec_heavy(GView<O, E, W> g, const W* 
         bool act = false;                                                                   \
         if (in) { s = g.row[i]; e = g.row[i + 1]; act = (e - s) > 0 && (e - s) <= HUB_DEG && g.vw[i] < max_allowed; } \
         W bw = 0; E bj = -1;                                                                \
-        if (act) heavy_edges<O, E, W>(g, max_allowed, s + lane, e, (E)G, bw, bj);          \
+        if (act) heavy_edges<O, E, W>(g, max_allowed, (Cursor<E>)s + lane, e, G, bw, bj);   \
         for (int m = G >> 1; m > 0; m >>= 1) {                                              \
             W w2 = shfl_xor(bw, m, G); E j2 = shfl_xor(bj, m, G);                           \
             argmax_merge<O, E, W>(bw, bj, w2, j2);                                          \
@@ -109,9 +110,9 @@ __global__ void __launch_bounds__(1024) k_hec_heavy_hub(GView<O, E, W> g, const 
         bool act = g.vw[i] < max_allowed;
         W bw = 0; E bj = -1;
         if (act)
-            for (E j = s + threadIdx.x; j < e; j += blockDim.x) {
+            for (Cursor<E> j = (Cursor<E>)s + threadIdx.x; j < (Cursor<E>)e; j += blockDim.x) {
                 O v = g.adj[j];
-                if (g.vw[v] < max_allowed) argmax_merge<O, E, W>(bw, bj, g.val[j], j);
+                if (g.vw[v] < max_allowed) argmax_merge<O, E, W>(bw, bj, g.val[j], (E)j);
             }
         for (int m = 16; m > 0; m >>= 1) {
             W w2 = shfl_xor(bw, m, 32); E j2 = shfl_xor(bj, m, 32);
@@ -301,8 +302,8 @@ __device__ __forceinline__ bool pick_skip(O u, const O* vcmap, const O* hn) {
 // four edges per round with the neighbour ids, weights and match states all
 // loaded before the first use.
 template <bool INITIAL, bool UNIFORM, class O, class E, class W>
-__device__ __forceinline__ void pick_edges(const GView<O, E, W>& g, const O* vcmap, uint32_t r, E j0, E e, E stride, int64_t& bw,
-                                           uint32_t& bh, int64_t& bj) {
+__device__ __forceinline__ void pick_edges(const GView<O, E, W>& g, const O* vcmap, uint32_t r, Cursor<E> j0, Cursor<E> e, Cursor<E> stride,
+                                           int64_t& bw, uint32_t& bh, int64_t& bj) {
     const O MAXV = ord_max<O>();
     for (; j0 < e; j0 += 4 * stride) {
         O v[4];
@@ -310,7 +311,7 @@ __device__ __forceinline__ void pick_edges(const GView<O, E, W>& g, const O* vcm
         bool ok[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            const E j = j0 + (E)u * stride;
+            const Cursor<E> j = j0 + u * stride;
             v[u] = j < e ? g.adj[j] : (O)-1;
             w[u] = (!UNIFORM && j < e) ? (int64_t)g.val[j] : 0;
         }
@@ -320,7 +321,7 @@ __device__ __forceinline__ void pick_edges(const GView<O, E, W>& g, const O* vcm
         for (int u = 0; u < 4; u++) {
             if (!ok[u]) continue;
             const uint32_t h = xorshift32((uint32_t)((uint64_t)v[u] + r));
-            const int64_t j = (int64_t)(j0 + (E)u * stride);
+            const int64_t j = (int64_t)(j0 + u * stride);
             if (pick_better(w[u], h, j, bw, bh, bj)) { bw = w[u]; bh = h; bj = j; }
         }
     }
@@ -341,7 +342,7 @@ __global__ void __launch_bounds__(BLOCK) k_pick_match(GView<O, E, W> g, const O*
             r = (uint32_t)jet_rng(seed, stream, (uint64_t)u);                               \
         }                                                                                   \
         int64_t bw = 0; uint32_t bh = 0; int64_t bj = -1;                                   \
-        if (act) pick_edges<INITIAL, UNIFORM, O, E, W>(g, vcmap, r, s + lane, e, (E)G, bw, bh, bj); \
+        if (act) pick_edges<INITIAL, UNIFORM, O, E, W>(g, vcmap, r, (Cursor<E>)s + lane, e, G, bw, bh, bj); \
         for (int m = G >> 1; m > 0; m >>= 1) {                                              \
             int64_t w2 = shfl_xor(bw, m, G); uint32_t h2 = shfl_xor(bh, m, G);              \
             int64_t j2 = shfl_xor(bj, m, G);                                                \
@@ -366,7 +367,7 @@ __global__ void __launch_bounds__(1024) k_pick_match_hub(GView<O, E, W> g, const
         if (!INITIAL && act) act = vcmap[u] == MAXV && hn[u] != MAXV;
         uint32_t r = (uint32_t)jet_rng(seed, stream, (uint64_t)u);
         int64_t bw = 0; uint32_t bh = 0; int64_t bj = -1;
-        if (act) pick_edges<INITIAL, UNIFORM, O, E, W>(g, vcmap, r, g.row[u] + threadIdx.x, g.row[u + 1], (E)blockDim.x, bw, bh, bj);
+        if (act) pick_edges<INITIAL, UNIFORM, O, E, W>(g, vcmap, r, (Cursor<E>)g.row[u] + threadIdx.x, g.row[u + 1], blockDim.x, bw, bh, bj);
         for (int m = 16; m > 0; m >>= 1) {
             int64_t w2 = shfl_xor(bw, m, 32); uint32_t h2 = shfl_xor(bh, m, 32); int64_t j2 = shfl_xor(bj, m, 32);
             if (pick_better(w2, h2, j2, bw, bh, bj)) { bw = w2; bh = h2; bj = j2; }
@@ -504,7 +505,9 @@ __global__ void __launch_bounds__(BLOCK) k_twin_hash(GView<O, E, W> g, const O* 
     {                                                                                       \
         uint64_t h = 0; O u = 0; E s = 0, e = 0;                                            \
         if (in) { u = list[x]; s = g.row[u]; e = g.row[u + 1]; if (e - s > HUB_DEG) e = s; } \
-        for (E j = s + lane; j < e; j += 32) { uint64_t y = id_hash<O>(g.adj[j], h64); h += y * y + y; } \
+        for (Cursor<E> j = (Cursor<E>)s + lane; j < (Cursor<E>)e; j += 32) {                \
+            uint64_t y = id_hash<O>(g.adj[j], h64); h += y * y + y;                         \
+        }                                                                                   \
         h = group_sum<uint64_t>(h, 32);                                                     \
         if (in && lane == 0 && g.row[u + 1] - s <= HUB_DEG) hashes[x] = h;                  \
     }
@@ -523,7 +526,10 @@ __global__ void __launch_bounds__(1024) k_twin_hash_hub(GView<O, E, W> g, const 
         if (vcmap[u] != ord_max<O>()) continue;
         E s = g.row[u], e = g.row[u + 1];
         uint64_t h = 0;
-        for (E j = s + threadIdx.x; j < e; j += blockDim.x) { uint64_t y = id_hash<O>(g.adj[j], h64); h += y * y + y; }
+        for (Cursor<E> j = (Cursor<E>)s + threadIdx.x; j < (Cursor<E>)e; j += blockDim.x) {
+            uint64_t y = id_hash<O>(g.adj[j], h64);
+            h += y * y + y;
+        }
         h = group_sum<uint64_t>(h, 32);
         if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = h;
         __syncthreads();

@@ -214,7 +214,7 @@ __device__ __forceinline__ void cta_for_row_edges(GView<O, E, W> g, const O* mem
     if (m1 - m0 <= FEW_MEMBERS) {
         for (O mi = m0; mi < m1; mi++) {
             O i = members[mi];
-            for (E j = g.row[i] + threadIdx.x; j < g.row[i + 1]; j += THREADS) f(j);
+            for (Cursor<E> j = (Cursor<E>)g.row[i] + threadIdx.x; j < (Cursor<E>)g.row[i + 1]; j += THREADS) f((E)j);
         }
         return;
     }
@@ -236,15 +236,15 @@ __device__ __forceinline__ void cta_for_row_edges(GView<O, E, W> g, const O* mem
             __syncthreads();
         }
         E total = s_pref[cnt - 1];
-        for (E t = threadIdx.x; t < total; t += THREADS) {
+        for (Cursor<E> t = threadIdx.x; t < (Cursor<E>)total; t += THREADS) {
             int lo = 0, hi = (int)cnt - 1;
             while (lo < hi) {
                 int mid = (lo + hi) >> 1;
-                if (s_pref[mid] > t) hi = mid; else lo = mid + 1;
+                if ((Cursor<E>)s_pref[mid] > t) hi = mid; else lo = mid + 1;
             }
             E before = lo > 0 ? s_pref[lo - 1] : 0;
             O i = s_mem[lo];
-            f(g.row[i] + (t - before));
+            f(g.row[i] + ((E)t - before));
         }
         __syncthreads();
     }
@@ -407,13 +407,13 @@ __global__ void __launch_bounds__(1024) k_contract_dense(GView<O, E, W> g, const
                 // few members (the usual case for dense rows): stride over each member's edges
                 for (O mi = m0; mi < m1; mi++) {
                     O i = members[mi];
-                    const E re = g.row[i + 1];
-                    for (E j0 = g.row[i] + threadIdx.x; j0 < re; j0 += 4 * (E)blockDim.x) {
+                    const Cursor<E> re = g.row[i + 1];
+                    for (Cursor<E> j0 = (Cursor<E>)g.row[i] + threadIdx.x; j0 < re; j0 += 4 * blockDim.x) {
                         O u[4];
                         W w[4];
 #pragma unroll
                         for (int q = 0; q < 4; q++) {
-                            const E j = j0 + q * (E)blockDim.x;
+                            const Cursor<E> j = j0 + q * blockDim.x;
                             u[q] = j < re ? g.adj[j] : (O)-1;
                             w[q] = j < re ? g.val[j] : (W)0;
                         }
@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(BLOCK) k_contract_copy_rows(O nc, const E* hro
         if (in) {                                                                           \
             const O c = (O)x;                                                               \
             const E hs = hrow[c], o = crow[c], cnt = crow[c + 1] - o;                      \
-            for (E t = lane; t < cnt; t += 32) { cadj[o + t] = skey[hs + t]; cval[o + t] = sval[hs + t]; } \
+            for (Cursor<E> t = lane; t < (Cursor<E>)cnt; t += 32) { cadj[o + t] = skey[hs + t]; cval[o + t] = sval[hs + t]; } \
         }                                                                                   \
     }
     JET_GROUP_LOOP(32, nc, CC_BODY)
@@ -511,7 +511,7 @@ __global__ void k_copy_chunk_rows(O nc, const E* crow, O* chunk_row) {
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x) {
         const E s = crow[c], t = crow[c + 1];
         if (t <= s) continue;
-        for (E j = (s + CT_COPY_CHUNK - 1) / CT_COPY_CHUNK; j * CT_COPY_CHUNK < t; j++) chunk_row[j] = (O)c;
+        for (int64_t j = ((int64_t)s + CT_COPY_CHUNK - 1) / CT_COPY_CHUNK; j * CT_COPY_CHUNK < (int64_t)t; j++) chunk_row[j] = (O)c;
     }
 }
 template <class O, class E, class W>
@@ -529,18 +529,18 @@ __global__ void __launch_bounds__(BLOCK) k_contract_copy(O nc, E mc, const O* ch
             const E hs = c < nc ? hrow[c] : (E)0;
             const E wend = r + 32 < (int64_t)nc ? crow[r + 32] : mc;
             const E lim = wend < e1 ? wend : e1;
-            for (E base = e; base < lim; base += 32) {
-                const E x = base + lane;
+            for (Cursor<E> base = e; base < (Cursor<E>)lim; base += 32) {
+                const Cursor<E> x = base + lane;
                 int lo = 0;
 #pragma unroll
                 for (int step = 16; step > 0; step >>= 1) {
                     const E v = __shfl_sync(0xffffffffu, os, lo + step);
-                    if (v <= x) lo += step;
+                    if ((Cursor<E>)v <= x) lo += step;
                 }
                 const E ro = __shfl_sync(0xffffffffu, os, lo);
                 const E rh = __shfl_sync(0xffffffffu, hs, lo);
-                if (x < lim) {
-                    const E src = rh + (x - ro);
+                if (x < (Cursor<E>)lim) {
+                    const E src = rh + ((E)x - ro);
                     cadj[x] = skey[src];
                     cval[x] = sval[src];
                 }
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(1024) k_hub_keys(GView<O, E, W> g, const O* ma
         for (O mi = moff[c]; mi < moff[c + 1]; mi++) {
             O i = members[mi];
             E rs = g.row[i], d = g.row[i + 1] - rs;
-            for (E t = threadIdx.x; t < d; t += blockDim.x) {
+            for (Cursor<E> t = threadIdx.x; t < (Cursor<E>)d; t += blockDim.x) {
                 O u = map[g.adj[rs + t]];
                 key[out + t] = u == c ? sentinel : (((uint64_t)x << nb) | (uint64_t)u);
                 val[out + t] = g.val[rs + t];

@@ -19,6 +19,12 @@
 namespace jetb {
 
 typedef int32_t part_t;
+// A cursor that strides over a row's entries passes the row's end, by up to
+// 4 * 1024 entries, before it stops, and offsets go up to the largest value of
+// their type: unsigned, the cursor has the bit that takes. (Signed, it wrapped
+// there to a negative offset, which lies before every end.)
+template <class E>
+using Cursor = std::make_unsigned_t<E>;
 static constexpr part_t NULL_PART = -1;     // src/jet_refiner.hpp:87
 static constexpr part_t HASH_RECLAIM = -2;  // src/jet_refiner.hpp:88
 static constexpr part_t NO_MOVE = -3;       // src/jet_refiner.hpp:89

@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_pstat_na(O n, const E* row, cons
         E s = row[x], e = row[x + 1];
         long long wsum = 0, fresh = 0;
         bool bad = false;
-        for (E j = s + lane; j < e; j += 32) {
+        for (Cursor<E> j = (Cursor<E>)s + lane; j < (Cursor<E>)e; j += 32) {
             int32_t p = part[adj[j]];
             if (p < 0 || p >= k) { bad = true; continue; }
             if (p == own) continue;
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_pstat_na(O n, const E* row, cons
             if (!(old & bit)) fresh++;
         }
         __syncwarp();
-        for (E j = s + lane; j < e; j += 32) {
+        for (Cursor<E> j = (Cursor<E>)s + lane; j < (Cursor<E>)e; j += 32) {
             int32_t p = part[adj[j]];
             if (p >= 0 && p < k && p != own) atomicAnd(&bitmap[wid][p >> 5], ~(1u << (p & 31)));
         }

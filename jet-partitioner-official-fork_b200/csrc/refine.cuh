@@ -200,16 +200,16 @@ __global__ void __launch_bounds__(THREADS) k_conn_thread(RefArgs<O, E, W> a, int
 #pragma unroll
         for (int s = 0; s < SET; s++) sk[s][t] = NULL_PART;
         int used = 0;
-        for (E j0 = rs; j0 < re; j0 += 8) {
+        for (Cursor<E> j0 = rs, je = re; j0 < je; j0 += 8) {
             O vb[8];
             W wb[8];
             part_t pb[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) vb[u] = j0 + u < re ? a.g.adj[j0 + u] : (O)0;
+            for (int u = 0; u < 8; u++) vb[u] = j0 + u < je ? a.g.adj[j0 + u] : (O)0;
 #pragma unroll
-            for (int u = 0; u < 8; u++) wb[u] = j0 + u < re ? a.g.val[j0 + u] : (W)0;
+            for (int u = 0; u < 8; u++) wb[u] = j0 + u < je ? a.g.val[j0 + u] : (W)0;
 #pragma unroll
-            for (int u = 0; u < 8; u++) pb[u] = j0 + u < re ? a.part[vb[u]] : NULL_PART;
+            for (int u = 0; u < 8; u++) pb[u] = j0 + u < je ? a.part[vb[u]] : NULL_PART;
 #pragma unroll
             for (int u = 0; u < 8; u++) {
                 part_t p = pb[u];
@@ -343,21 +343,22 @@ __device__ __forceinline__ void smem_table_flush(const part_t* keys, const W* va
 // (the part gather depends on the neighbour id load).  Returns the slots this
 // thread claimed.
 template <class O, class E, class W>
-__device__ __forceinline__ int table_add_edges(const RefArgs<O, E, W>& a, part_t* keys, W* vals, part_t cap, E rs, E re, int t,
+__device__ __forceinline__ int table_add_edges(const RefArgs<O, E, W>& a, part_t* keys, W* vals, part_t cap, E rs, E end, int t,
                                                int nt) {
+    const Cursor<E> re = end;
     int mine = 0;
-    for (E j0 = rs + t; j0 < re; j0 += 4 * (E)nt) {
+    for (Cursor<E> j0 = (Cursor<E>)rs + t; j0 < re; j0 += 4 * nt) {
         O v[4];
         W w[4];
         part_t p[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            E j = j0 + (E)u * nt;
+            const Cursor<E> j = j0 + u * nt;
             v[u] = j < re ? a.g.adj[j] : (O)0;
             w[u] = j < re ? a.g.val[j] : (W)0;
         }
 #pragma unroll
-        for (int u = 0; u < 4; u++) p[u] = j0 + (E)u * nt < re ? a.part[v[u]] : NULL_PART;
+        for (int u = 0; u < 4; u++) p[u] = j0 + u * nt < re ? a.part[v[u]] : NULL_PART;
 #pragma unroll
         for (int u = 0; u < 4; u++)
             if (p[u] != NULL_PART) mine += smem_table_add<W>(keys, vals, cap, a.k, p[u], w[u], &a.dev->err, a.narrow);
@@ -493,18 +494,18 @@ __device__ __forceinline__ void conn_warp_row(const RefArgs<O, E, W>& a, O i, E 
         __syncwarp();
         return;
     }
-    for (E j0 = rs + lane; j0 < re; j0 += 4 * 32) {
+    for (Cursor<E> j0 = (Cursor<E>)rs + lane, je = re; j0 < je; j0 += 4 * 32) {
         O v[4];
         W w[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            E j = j0 + (E)u * 32;
-            v[u] = j < re ? a.g.adj[j] : (O)0;
-            w[u] = j < re ? a.g.val[j] : (W)0;
+            const Cursor<E> j = j0 + u * 32;
+            v[u] = j < je ? a.g.adj[j] : (O)0;
+            w[u] = j < je ? a.g.val[j] : (W)0;
         }
         part_t p[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) p[u] = j0 + (E)u * 32 < re ? a.part[v[u]] : NULL_PART;
+        for (int u = 0; u < 4; u++) p[u] = j0 + u * 32 < je ? a.part[v[u]] : NULL_PART;
 #pragma unroll
         for (int u = 0; u < 4; u++)
             if (p[u] != NULL_PART) acc_add<W>(&vals[p[u]], w[u], a.narrow);
@@ -558,18 +559,18 @@ __device__ __forceinline__ void conn_block_row_priv(const RefArgs<O, E, W>& a, O
     const int nw = (int)(blockDim.x >> 5), wid = threadIdx.x >> 5;
     if (threadIdx.x == 0) *s_used = 0;
     W* my = acc + wid * a.k;
-    for (E j0 = rs + threadIdx.x; j0 < re; j0 += 4 * (E)blockDim.x) {
+    for (Cursor<E> j0 = (Cursor<E>)rs + threadIdx.x, je = re; j0 < je; j0 += 4 * blockDim.x) {
         O v[4];
         W w[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            E j = j0 + (E)u * blockDim.x;
-            v[u] = j < re ? a.g.adj[j] : (O)0;
-            w[u] = j < re ? a.g.val[j] : (W)0;
+            const Cursor<E> j = j0 + u * blockDim.x;
+            v[u] = j < je ? a.g.adj[j] : (O)0;
+            w[u] = j < je ? a.g.val[j] : (W)0;
         }
 #pragma unroll
         for (int u = 0; u < 4; u++)
-            if (j0 + (E)u * blockDim.x < re) acc_add<W>(&my[a.part[v[u]]], w[u], a.narrow);
+            if (j0 + u * blockDim.x < je) acc_add<W>(&my[a.part[v[u]]], w[u], a.narrow);
     }
     __syncthreads();
     // merge: one thread per part sums the nw arrays (consecutive parts on
@@ -1131,7 +1132,8 @@ struct WalkNothing {
 // pregains, then their destinations and parts where needed) issued before
 // the first use.
 template <class O, class E, class W>
-__device__ __forceinline__ W afterburn_edges(const RefArgs<O, E, W>& a, O i, W igain, part_t p, part_t best, E j0, E e, E stride) {
+__device__ __forceinline__ W afterburn_edges(const RefArgs<O, E, W>& a, O i, W igain, part_t p, part_t best, Cursor<E> j0, Cursor<E> e,
+                                             Cursor<E> stride) {
     W ch = 0;
     for (; j0 < e; j0 += 4 * stride) {
         O v[4];
@@ -1140,7 +1142,7 @@ __device__ __forceinline__ W afterburn_edges(const RefArgs<O, E, W>& a, O i, W i
         bool take[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            const E j = j0 + (E)u * stride;
+            const Cursor<E> j = j0 + u * stride;
             v[u] = j < e ? a.g.adj[j] : (O)-1;
             w[u] = j < e ? a.g.val[j] : (W)0;
         }
@@ -1174,7 +1176,7 @@ __device__ __forceinline__ void d_afterburn(RefArgs<O, E, W> a) {
             igain = a.pregain[i]; p = a.part[i]; best = a.dest[i];                          \
         }                                                                                   \
         W ch = 0;                                                                           \
-        if (act) ch = afterburn_edges<O, E, W>(a, i, igain, p, best, s + lane, e, (E)G);   \
+        if (act) ch = afterburn_edges<O, E, W>(a, i, igain, p, best, (Cursor<E>)s + lane, e, G); \
         ch = group_sum<W>(ch, G);                                                           \
         bool keep = act && lane == 0 && igain + ch >= 0;                                    \
         if (keep) a.lock[i] = 1;                                                            \
@@ -1256,7 +1258,7 @@ __device__ __forceinline__ void d_afterburn_hub(RefArgs<O, E, W> a) {
         W igain = a.pregain[i];
         part_t p = a.part[i], best = a.dest[i];
         W ch = 0;
-        ch = afterburn_edges<O, E, W>(a, i, igain, p, best, a.g.row[i] + threadIdx.x, a.g.row[i + 1], (E)blockDim.x);
+        ch = afterburn_edges<O, E, W>(a, i, igain, p, best, (Cursor<E>)a.g.row[i] + threadIdx.x, a.g.row[i + 1], blockDim.x);
         ch = group_sum<W>(ch, 32);
         if ((threadIdx.x & 31) == 0) part_sum[threadIdx.x >> 5] = ch;
         __syncthreads();
@@ -2307,12 +2309,12 @@ __device__ __forceinline__ void conn_add(const RefArgs<O, E, W>& a, O v, part_t 
 // round, every load issued before the first use, and only unmarked ones
 // written, so that few lines get dirty.
 template <class O, class E, class W>
-__device__ __forceinline__ void mark_edges(const RefArgs<O, E, W>& a, E j0, E re, E stride) {
+__device__ __forceinline__ void mark_edges(const RefArgs<O, E, W>& a, Cursor<E> j0, Cursor<E> re, Cursor<E> stride) {
     for (; j0 < re; j0 += 4 * stride) {
         O v[4];
         uint8_t mk[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) v[u] = j0 + (E)u * stride < re ? a.g.adj[j0 + (E)u * stride] : (O)-1;
+        for (int u = 0; u < 4; u++) v[u] = j0 + u * stride < re ? a.g.adj[j0 + u * stride] : (O)-1;
 #pragma unroll
         for (int u = 0; u < 4; u++) mk[u] = v[u] >= 0 ? a.mark[v[u]] : (uint8_t)1;
 #pragma unroll
@@ -2352,8 +2354,10 @@ __device__ __forceinline__ void d_apply_moves(const RefArgs<O, E, W>& a, W* hs) 
             if (e - s > HUB_DEG) { O h = atomic_add(&a.dev->nmoves_hub, (O)1); a.moves_hub[h] = i; } \
         }                                                                                   \
         if (in && e - s <= HUB_DEG) {                                                       \
-            if (large) mark_edges<O, E, W>(a, s + lane, e, (E)G);                           \
-            else for (E j = s + lane; j < e; j += G) conn_sub<O, E, W>(a, a.g.adj[j], p, a.g.val[j]); \
+            if (large) mark_edges<O, E, W>(a, (Cursor<E>)s + lane, e, G);                   \
+            else                                                                            \
+                for (Cursor<E> j = (Cursor<E>)s + lane; j < (Cursor<E>)e; j += G)           \
+                    conn_sub<O, E, W>(a, a.g.adj[j], p, a.g.val[j]);                        \
         }                                                                                   \
     }
     JET_GROUP_LOOP(G, count, APPLY_BODY)
@@ -2429,9 +2433,9 @@ __device__ __forceinline__ void d_apply_hub(const RefArgs<O, E, W>& a) {
     for (O x = blockIdx.x; x < count; x += gridDim.x) {
         const O i = a.moves_hub[x];
         const part_t p = a.dest[i];  // the part it left
-        const E re = a.g.row[i + 1];
-        E j = a.g.row[i] + threadIdx.x;
-        if (large) mark_edges<O, E, W>(a, j, re, (E)blockDim.x);
+        const Cursor<E> re = a.g.row[i + 1];
+        Cursor<E> j = (Cursor<E>)a.g.row[i] + threadIdx.x;
+        if (large) mark_edges<O, E, W>(a, j, re, blockDim.x);
         else for (; j < re; j += blockDim.x) conn_sub<O, E, W>(a, a.g.adj[j], p, a.g.val[j]);
     }
 }
@@ -2442,7 +2446,7 @@ __global__ void __launch_bounds__(1024) k_apply_hub(RefArgs<O, E, W> a) { d_appl
 // share of the cut change: where the neighbour moved too, what the move
 // changed in the connection to its new part less that to its old one.
 template <class O, class E, class W>
-__device__ __forceinline__ W add_edge(const RefArgs<O, E, W>& a, part_t from, part_t to, uint32_t now, E j) {
+__device__ __forceinline__ W add_edge(const RefArgs<O, E, W>& a, part_t from, part_t to, uint32_t now, Cursor<E> j) {
     const O v = a.g.adj[j];
     const W w = a.g.val[j];
     const bool moved = a.stamp[v] == now;
@@ -2464,7 +2468,8 @@ __device__ __forceinline__ void d_update_add(const RefArgs<O, E, W>& a) {
             const E s = a.g.row[i], e = a.g.row[i + 1];                                     \
             const part_t from = a.dest[i], to = a.part[i];                                  \
             if (e - s <= HUB_DEG)                                                           \
-                for (E j = s + lane; j < e; j += G) c2 += add_edge<O, E, W>(a, from, to, now, j); \
+                for (Cursor<E> j = (Cursor<E>)s + lane; j < (Cursor<E>)e; j += G)           \
+                    c2 += add_edge<O, E, W>(a, from, to, now, j);                           \
         }                                                                                   \
     }
     JET_GROUP_LOOP(G, count, ADD_BODY)
@@ -2494,8 +2499,8 @@ __device__ __forceinline__ void d_update_add_hub(const RefArgs<O, E, W>& a) {
     for (O x = blockIdx.x; x < count; x += gridDim.x) {
         const O i = a.moves_hub[x];
         const part_t from = a.dest[i], to = a.part[i];
-        const E re = a.g.row[i + 1];
-        for (E j = a.g.row[i] + threadIdx.x; j < re; j += blockDim.x) c2 += add_edge<O, E, W>(a, from, to, now, j);
+        const Cursor<E> re = a.g.row[i + 1];
+        for (Cursor<E> j = (Cursor<E>)a.g.row[i] + threadIdx.x; j < re; j += blockDim.x) c2 += add_edge<O, E, W>(a, from, to, now, j);
     }
     c2 = group_sum<W>(c2, 32);
     if ((threadIdx.x & 31) == 0 && c2) atomic_add(&a.dev->cut2, c2);
@@ -2793,7 +2798,8 @@ __global__ void __launch_bounds__(BLOCK) k_total_cut(GView<O, E, W> g, const par
     {                                                                                       \
         if (in) {                                                                           \
             O i = (O)x; part_t pi = part[i];                                                \
-            for (E j = g.row[i] + lane; j < g.row[i + 1]; j += G) if (part[g.adj[j]] != pi) acc += g.val[j]; \
+            const Cursor<E> e = g.row[i + 1];                                               \
+            for (Cursor<E> j = (Cursor<E>)g.row[i] + lane; j < e; j += G) if (part[g.adj[j]] != pi) acc += g.val[j]; \
         }                                                                                   \
     }
     JET_GROUP_LOOP(G, g.n, CUT_BODY)

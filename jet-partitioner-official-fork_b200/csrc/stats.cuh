@@ -120,19 +120,19 @@ __global__ void __launch_bounds__(BLOCKWIDE ? 1024 : BLOCK) k_pstat_long(GView<O
         for (int w = t; w < words; w += nt) bm[w] = 0;
         if (BLOCKWIDE) __syncthreads(); else __syncwarp();
         W acc = 0;
-        const E re = g.row[i + 1];
-        for (E j0 = g.row[i] + t; j0 < re; j0 += 4 * (E)nt) {
+        const Cursor<E> re = g.row[i + 1];
+        for (Cursor<E> j0 = (Cursor<E>)g.row[i] + t; j0 < re; j0 += 4 * nt) {
             O v[4];
             W w[4];
             part_t p[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                const E j = j0 + (E)u * nt;
+                const Cursor<E> j = j0 + u * nt;
                 v[u] = j < re ? g.adj[j] : (O)0;
                 w[u] = j < re ? g.val[j] : (W)0;
             }
 #pragma unroll
-            for (int u = 0; u < 4; u++) p[u] = j0 + (E)u * nt < re ? part[v[u]] : own;
+            for (int u = 0; u < 4; u++) p[u] = j0 + u * nt < re ? part[v[u]] : own;
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 if (p[u] == own || p[u] < 0 || p[u] >= k) continue;

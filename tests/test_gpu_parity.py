@@ -815,3 +815,49 @@ def test_level_drivers_64_bit(jet, graphs, orc, drivers, tier, k):
     want, wcut, _ = orc.partition(orc.G.from_csr(g), k, alg=0, imb=1.03, seed=3)
     part, cut = _partition_with(jet, mask, tier, cfg, g, 3)
     assert cut == wcut and np.array_equal(part, want)
+
+
+def test_rows_that_end_at_the_largest_offset(jet, graphs):
+    """An i32 graph of 2^31 - 1 entries: cursors over its last row step past
+    the largest 32-bit offset. Statistics, tables and contraction equal counts
+    of the rows' entries (entry j names vertex j mod 1009)."""
+    m, per, v, k, members = 2 ** 31 - 1, 16384, 1009, 64, 32
+    n = (m + 1) // per
+    dev = "cuda"
+    row = torch.arange(n + 1, device=dev, dtype=torch.int64) * per
+    row[n] = m
+    adj = torch.arange(m, device=dev, dtype=torch.int32).remainder_(v)
+    g = graphs.CSRGraph(n, row.to(torch.int32), adj, torch.ones(m, dtype=torch.int32, device=dev),
+                        torch.ones(n, dtype=torch.int32, device=dev), True, "i32")
+    part = (torch.arange(n, device=dev, dtype=torch.int32) * 7) % k
+    # entries of row i that name x: whole periods, and the rest from the row's first id on
+    first, length = (row[:-1] % v)[:, None], (row[1:] - row[:-1])[:, None]
+    ids = torch.arange(v, device=dev)[None, :]
+    times = (length // v + ((ids - first) % v < length % v)).to(torch.int32)
+    to_part = torch.zeros(n, k, dtype=torch.int32, device=dev).index_add_(1, part[:v].long(), times)
+    own = to_part.gather(1, part[:, None].long())[:, 0]
+    out = length[:, 0] - own
+    per_part = torch.zeros(k, dtype=torch.int64, device=dev).index_add_(0, part.long(), out)
+    sizes = torch.bincount(part, minlength=k)
+    want = [int(out.sum()) // 2, int(per_part.max()), int((to_part > 0).sum() - (own > 0).sum()), int(sizes.max()), int(sizes.min()), n]
+    assert jet.pstat(g, part, k) == want
+    assert jet.pstat_noalloc(g, part, k) == want
+
+    off, ent, val, size = jet.conn_build(g, part, k)
+    # every row has every part, so tables are direct: k slots, a part at its own
+    assert torch.equal(off, torch.arange(n + 1, device=dev, dtype=torch.int32) * k) and bool((size == k).all())
+    assert torch.equal(ent.view(n, k), torch.arange(k, device=dev, dtype=torch.int32).expand(n, k))
+    assert torch.equal(val.view(n, k), to_part)
+    del off, ent, val, size, to_part
+
+    nc = n // members
+    cmap = torch.arange(n, device=dev, dtype=torch.int32) // members
+    c = jet.contract(g, cmap, nc)
+    coarse = torch.zeros(nc, (v - 1) // members + 1, dtype=torch.int32, device=dev)
+    coarse.index_add_(1, cmap[:v].long(), times.view(nc, members, v).sum(1, dtype=torch.int32))
+    at = torch.arange(coarse.shape[1], device=dev)
+    coarse[at, at] = 0
+    keep = coarse > 0
+    assert torch.equal(c.row[1:] - c.row[:-1], keep.sum(1, dtype=torch.int32))
+    assert torch.equal(c.adj, keep.nonzero()[:, 1].to(torch.int32)) and torch.equal(c.val, coarse[keep])
+    assert bool((c.vw == members).all())
