@@ -796,7 +796,7 @@ struct Refiner {
     }
     static bool long_rows(const Level<O, E, W>& L) { return long_rows((int64_t)L.n, (int64_t)L.m, (int64_t)L.max_deg, (int64_t)L.n_hub); }
     bool cta_eligible(const Level<O, E, W>& L) const {
-        int64_t cap = (use_cluster && !batch_thread() && cluster_size(L) > 0) ? cta_prefer_n() : CTA_MAX_N;
+        int64_t cap = (use_cluster && !batch_thread() && cluster_size() > 0) ? cta_prefer_n() : CTA_MAX_N;
         return use_cta && (int64_t)L.n <= cap && (int64_t)L.m <= CTA_MAX_M && k <= CTA_MAX_K;
     }
 
@@ -942,22 +942,22 @@ struct Refiner {
     static constexpr int64_t CLUSTER_MAX_N_MANY = (int64_t)1 << 15;
     static constexpr int64_t CLUSTER_MAX_M = (int64_t)1 << 21;
     // CTAs in the level cluster: 16 where the device allows it, else 8, 0 if
-    // no cluster of 1024-thread CTAs with this shared memory fits.
+    // no cluster of 1024-thread CTAs fits. Asked once, with the most shared memory
+    // that a level may take: one such CTA fills an SM's registers, so less
+    // changes nothing (asked for each level, it took 50 us of a 256 x 256 grid's call).
     mutable int cluster_cache = -1;
-    mutable size_t cluster_cache_smem = 0;
-    int cluster_size(const Level<O, E, W>& L) const {
-        const size_t smem = coop_smem(L);
-        if (cluster_cache >= 0 && cluster_cache_smem == smem) return cluster_cache;
-        cluster_cache_smem = smem;
-        cluster_cache = [smem] {
+    int cluster_size() const {
+        if (cluster_cache >= 0) return cluster_cache;
+        cluster_cache = [] {
             const void* f = (const void*)k_level_coop<true, false, false, O, E, W>;
-            if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem(f)) != cudaSuccess) return 0;
+            const int smem = max_dynamic_smem(f);
+            if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 0;
             cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             for (int want : {16, 8}) {
                 cudaLaunchConfig_t cfg = {};
                 cfg.gridDim = dim3(want);
                 cfg.blockDim = dim3(CTA_THREADS);
-                cfg.dynamicSmemBytes = smem;
+                cfg.dynamicSmemBytes = (size_t)smem;
                 cudaLaunchAttribute at;
                 at.id = cudaLaunchAttributeClusterDimension;
                 at.val.clusterDim.x = want;
@@ -976,7 +976,7 @@ struct Refiner {
     bool cluster_eligible(const Level<O, E, W>& L) const {
         return use_cluster && !cta_eligible(L) && (int64_t)L.n <= cluster_max_n() && (int64_t)L.m <= cluster_max_m() &&
                k <= LEVEL_MAX_K && table_width(L) <= WARP_TABLE &&
-               coop_smem(L) + coop_static_smem() <= (size_t)device_info().max_smem_optin && cluster_size(L) > 0;
+               coop_smem(L) + coop_static_smem() <= (size_t)device_info().max_smem_optin && cluster_size() > 0;
     }
 
     // The whole level loop as one persistent launch: a single cluster
@@ -994,7 +994,7 @@ struct Refiner {
                                                : (const void*)k_level_coop<false, false, false, O, E, W>;
         int grid = 0;
         if (cluster) {
-            grid = cluster_size(L);
+            grid = cluster_size();
         } else {
             JET_CUDA(cudaFuncSetAttribute(grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem(grid_kernel)));
             int per_sm = 0;
