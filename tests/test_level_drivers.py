@@ -160,3 +160,29 @@ def test_large_levels_of_long_rows_stay_level_graphs(jet, graphs, scale, degree,
     jet.prof_phases(True)
     jet.refine_level(g, part, 16, 1.10)
     assert {d for d, p in jet.prof_phases(False).items() if p} == loops
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tier,wide", [("i32", False), ("big", True)])
+def test_row_walk_many_rounds(jet, graphs, orc, tier, wide):
+    """A level of the persistent grid whose first iteration has more moves
+    than 32 for each of its warps: the walks over the rows of candidates and
+    moves take several rounds. A random partition of a 700 x 700 mesh; the
+    refined level equals the oracle's."""
+    g = graphs.grid2d(700, 700, weighted=True, seed=2).as_tier(tier)
+    if wide:
+        g.val = g.val * (2 ** 31 // int(g.val.sum()) + 1)
+    og = orc.G.from_csr(g)
+    part = torch.randint(0, 5, (g.n,), generator=torch.Generator().manual_seed(4), dtype=torch.int32)
+    warps = 32 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert orc.refine_iters(og, part.numpy(), 5, 1.10, 0.75, 1)["moves"][0] > 32 * warps
+    want, wcut, _ = orc.refine_level(og, part.numpy(), 5, 1.10)
+    prev = jet.set_refine_drivers(jet.DRIVER_COOP | jet.DRIVER_GRAPH | jet.DRIVER_REB_QUEUE)
+    try:
+        jet.prof_phases(True)
+        got, cut, _ = jet.refine_level(g.to("cuda"), part.cuda(), 5, 1.10)
+        ran = {d for d, p in jet.prof_phases(False).items() if p}
+    finally:
+        jet.set_refine_drivers(prev)
+    assert ran == {"coop"}
+    assert cut == wcut and (got.cpu().numpy() == want).all()
