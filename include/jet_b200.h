@@ -270,9 +270,10 @@ int jet_prof_enable(int on);
  * times the phase ran; on = 0 copies out[6 * 24] and stops.  Layout:
  * driver d (0 one CTA, 1 cluster, 2 cooperative) at out[48 d]: cycles of
  * phases 0-23, then their counts.  Phases: 0 LP select, 1 afterburner,
- * 2 hub afterburner, 3 rebalance prep, 4 rebalance select, 5 bucket scan,
- * 6 candidate sort, 7 eviction, 8 strong tail, 9 apply, 10 update subtract,
- * 11 update add + mark, 12 row rebuild, 13 cut change, 14 control, 15 copy,
+ * 2 hub afterburner, 4 rebalance select, 5 bucket scan, 6 candidate sort,
+ * 7 eviction, 9 moves with the subtract pass (or marks), 10 the same for hub
+ * rows, 11 add pass with the cut change and the close, 12 row rebuild, 13 cut
+ * change after a rebuild, 14 control, 15 copy (3 and 8 are not recorded),
  * 16 cookie cutter, 17 strong destinations, 18 strong re-draws, 19 sorted
  * weight prefix. */
 int jet_prof_phases(int on, uint64_t* out);

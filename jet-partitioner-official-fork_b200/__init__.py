@@ -71,8 +71,9 @@ def metis_call_stats() -> dict:
     return dict(helper_calls=out[0], helper_failures=out[1], inprocess_calls=out[2], helpers=out[3],
                 helpers_unavailable=bool(out[4]), helper_metis_errors=out[5])
 
-PHASES = ["lp_select", "afterburn", "afterburn_hub", "reb_prep", "reb_select", "bucket_scan", "cand_sort", "evict",
-          "strong_tail", "apply", "update_sub", "update_add", "rebuild", "cut", "control", "copy", "cookie",
+# (None: a slot that nothing records)
+PHASES = ["lp_select", "afterburn", "afterburn_hub", None, "reb_select", "bucket_scan", "cand_sort", "evict",
+          None, "apply", "update_sub", "update_add", "rebuild", "cut", "control", "copy", "cookie",
           "strong_first", "redraw", "weight_scan"]
 
 

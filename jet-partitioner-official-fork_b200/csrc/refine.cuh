@@ -127,9 +127,11 @@ struct RefArgs {
 // only; nothing is recorded without a.pclk).  Slots [base + id] hold cycles,
 // [base + PHASE_SLOTS + id] the number of times the phase ran.
 static constexpr int PHASE_SLOTS = 24;
+// (3 and 8 are free: the block that closes an iteration prepares the next
+// rebalance, and the strong tail's steps have slots of their own)
 enum PhaseId : int {
-    PH_LP_SELECT = 0, PH_AFTERBURN, PH_AFTERBURN_HUB, PH_REB_PREP, PH_REB_SELECT, PH_REB_SCAN, PH_REB_SORT, PH_REB_EVICT,
-    PH_STRONG_TAIL, PH_APPLY, PH_UPDATE_SUB, PH_UPDATE_ADD, PH_REBUILD, PH_CUT, PH_CTL, PH_COPY,
+    PH_LP_SELECT = 0, PH_AFTERBURN, PH_AFTERBURN_HUB, PH_REB_SELECT = 4, PH_REB_SCAN, PH_REB_SORT, PH_REB_EVICT,
+    PH_APPLY = 9, PH_UPDATE_SUB, PH_UPDATE_ADD, PH_REBUILD, PH_CUT, PH_CTL, PH_COPY,
     PH_COOKIE, PH_STRONG_FIRST, PH_REDRAW, PH_WEIGHT_SCAN, PH_COUNT
 };
 struct PhaseClock {
@@ -846,11 +848,13 @@ __device__ __forceinline__ void d_lp_select_thread(RefArgs<O, E, W> a) {
 // them per lane before the first use, finishes the light ones and collects
 // the others in shared memory; those are then dealt to the lanes, several to
 // a vertex where few are left (PassDeal).
-// These are the grid kernels' forms: on the 2.1 M-vertex level of the 128^3
-// mesh an iteration went from 128 to 118 us, on R-MAT 2^24's finest level from
-// 5.69 to 5.47 ms. The persistent level loops keep one vertex per thread: their
-// levels have one to two rounds, nothing to overlap, and the longer code cost
-// them 2-3 us a pass (one CTA: LP select 2.8 -> 6.1 us, classification 1.1 -> 3.0).
+// These are the forms of the grid kernels and of the persistent grid's larger
+// levels (PASS: above two vertices per thread): on the 2.1 M-vertex level of the
+// 128^3 mesh an iteration went from 128 to 118 us, on R-MAT 2^24's finest level
+// from 5.69 to 5.47 ms. The one-CTA and cluster loops and the grid's smaller
+// levels keep one vertex per thread: they have one to two rounds, nothing to
+// overlap, and the longer code cost them 2-3 us a pass (one CTA: LP select 2.8 ->
+// 6.1 us, classification 1.1 -> 3.0).
 // `list`: 32 * PASS_U bytes of shared memory per warp.
 static constexpr int PASS_U = 4;
 static constexpr int PASS_LIST = 32 * PASS_U;

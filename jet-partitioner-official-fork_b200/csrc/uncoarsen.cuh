@@ -854,9 +854,12 @@ struct Refiner {
     // geometric graph of 800,000 (8 M entries) into 32 92 and 61, 128^3 mesh's
     // 749,582-vertex level (7.5 M) into 64 103 and 88, 100^3 mesh into 256 103 and
     // 90, a 504,000-vertex mesh into 300 104 and 78; but 128^3's finest level (2.1 M,
-    // 12.5 M entries) 107 and 110-116. With many parts a rebalance queues more
+    // 12.5 M entries) 107 and 110-116. With many parts a rebalance can queue more
     // candidates than the grid's block orders (COOP_QUEUE_KEYS) and takes the
     // full sort: 717,120 vertices into 768 parts 111 and 146 (387,988: 114 and 107).
+    // The bound for more than 512 parts rests on that mesh alone and is on the safe
+    // side: 600,000-vertex levels ran 106 and 79 (mesh, 600 parts), 118 and 86
+    // (1,000), 114 and 64, 119 and 66 (geometric graph).
     // Nor do levels of long rows gain above that bound (R-MAT 2^19 into 64 parts:
     // finest level 365 and 489), and with 64-bit weights they lose from fewer
     // entries on (R-MAT 2^19's levels of 6-8 M entries 434-604 in the graph and 590-749).
@@ -864,11 +867,11 @@ struct Refiner {
     static constexpr int64_t COOP_MAX_N_MANY = (int64_t)1 << 18;
     static constexpr int64_t COOP_MAX_M_LONG = (int64_t)1 << 22;
     // Parts up to which the persistent loops take a level whose rows fit the
-    // warps' shared-memory tables. 717k-vertex mesh into 768 parts: its levels
-    // of 1,323-61,159 vertices ran 98-297 us per iteration as level graphs
-    // and run 89-171 on the cluster (the whole call 161.6 -> 151.0 ms, of
-    // which Metis 73); beyond about 1,000 parts the bucket arrays (50 per part
-    // and section) outgrow the blocks' shared memory and the gain.
+    // warps' shared-memory tables. All refinement of 60,000 vertices as level
+    // graphs and here, ms: mesh into 513, 700 and 1,000 parts 22.5 and 12.6, 23.6
+    // and 14.2, 27.1 and 17.9; geometric graph 19.3 and 10.5, 16.4 and 8.8, 20.8
+    // and 12.5. Beyond about 1,000 parts the bucket arrays (50 per part and
+    // section) outgrow the blocks' shared memory.
     static constexpr part_t LEVEL_MAX_K = 1024;
     static constexpr int64_t COOP_MAX_M = (int64_t)1 << 23;
     size_t coop_smem(const Level<O, E, W>& L) const {
@@ -886,9 +889,10 @@ struct Refiner {
         return ((keys > rs ? keys : rs) + 15) & ~(size_t)15;
     }
     // rebalance candidates block 0 of the persistent grid orders in shared memory
-    // (2048 keys hold every queue seen on meshes and geometric graphs at
-    // these sizes; more shared memory here would come out of the L1 cache
-    // the loop's global accesses hit)
+    // (2048 keys hold the queues of meshes into 64 parts, 886 at most; many parts
+    // and power-law levels overflow them and take the full sort. More shared
+    // memory here would come out of the L1 cache that the loop's global
+    // accesses hit)
     static constexpr int COOP_QUEUE_KEYS = 2048;
     int coop_qcap() const { return COOP_QUEUE_KEYS; }
     // Bucket offsets that every block of a cluster or grid loop keeps in shared
@@ -935,9 +939,11 @@ struct Refiner {
     // power-law levels of tens of millions of entries.
     static constexpr int64_t CLUSTER_MAX_N = (int64_t)1 << 16;
     // (more parts than this: every block reads and scans 50 bucket totals per
-    // part, which 16 blocks do no faster than 148; 768 parts, 33,618 vertices 117
-    // us per iteration in the cluster and 107 in the grid, 61,251 vertices 133 and
-    // 109. 32 parts, 65,536 vertices: 36 and 41)
+    // part, which 16 blocks do no faster than 148. us per iteration in the
+    // cluster and in the grid: 768 parts, mesh of 33,618 vertices 117 and 107,
+    // 61,251 133 and 109; 59,319 into 700 and 1,000 59 and 55, 62 and 59; geometric
+    // graph of 60,000 54 and 52, 59 and 56. From 300 to 513 parts, 59,319 and
+    // 60,000 vertices: within 2 of one another; 32 parts, 65,536: 36 and 41)
     static constexpr part_t MANY_PARTS = 512;
     static constexpr int64_t CLUSTER_MAX_N_MANY = (int64_t)1 << 15;
     static constexpr int64_t CLUSTER_MAX_M = (int64_t)1 << 21;
