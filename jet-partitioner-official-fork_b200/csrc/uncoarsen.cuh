@@ -778,21 +778,24 @@ struct Refiner {
     static int64_t cluster_max_m() { static const int64_t v = bound("JET_PERSISTENT_MAX_M", CLUSTER_MAX_M); return v; }
     static int64_t coop_max_m(const Level<O, E, W>& L) {
         static const int64_t v = bound("JET_PERSISTENT_MAX_M", UNSET);
-        return v != UNSET ? v : (sizeof(W) == 8 && long_rows(L) ? COOP_MAX_M_LONG : COOP_MAX_M);
+        return v != UNSET ? v : (sizeof(W) == 8 && (L.n_hub > 0 || long_rows(L)) ? COOP_MAX_M_LONG : COOP_MAX_M);
     }
     // Levels whose rows the persistent loops give a group of lanes each, instead
     // of walking them as one sequence per warp (warp_rows): rows of very uneven
     // length, where a warp that draws several long ones holds up the phase (hub
-    // rows, or a mean of 32 edges and a longest row of four times that), and small
-    // dense levels, whose every row fills the warps by itself (a mean of 32 and
-    // of a sixteenth of the vertices). us per iteration as walks and in groups:
-    // R-MAT levels into 32 parts, 26,710 vertices (mean 62) 494 and 301, 8,593
-    // (173) 308 and 222, 480 (209) 101 and 91; the first with 64-bit weights 807
-    // and 527; HEC's R-MAT level of 22,427 (91) 1,296 and 732. Even rows are
-    // better walked: geometric graphs of 15,058 vertices (mean 180) 149 and 159,
-    // 33,258 (42) 108 and 110, 132,498 (13) 45 and 54.
+    // rows and a mean of 14 edges, or a mean of 32 and a longest row of four times
+    // that), and small dense levels, whose every row fills the warps by itself (a
+    // mean of 32 and of a sixteenth of the vertices). us per iteration as walks
+    // and in groups: R-MAT levels into 32 parts, 26,710 vertices (mean 62) 494 and
+    // 301, 8,593 (173) 308 and 222, 480 (209) 101 and 91; the first with 64-bit
+    // weights 807 and 527, R-MAT 2^16 (14.6) with them 573 and 453; HEC's R-MAT
+    // level of 22,427 (91) 1,296 and 732. Even rows are better walked: geometric
+    // graphs of 15,058 vertices (mean 180) 149 and 159, 33,258 (42) 108 and 110,
+    // 132,498 (13) 45 and 54. So are hubs among short rows: levels of 540,649
+    // vertices (mean 2) and 556,538 (5.6) of a matching hierarchy of R-MAT 2^20 88
+    // and 168, 229 and 465.
     static bool long_rows(int64_t n, int64_t m, int64_t max_deg, int64_t n_hub) {
-        return n_hub > 0 || (m >= 32 * n && (max_deg * n >= 4 * m || 16 * m >= n * n));
+        return (n_hub > 0 && m >= 14 * n) || (m >= 32 * n && (max_deg * n >= 4 * m || 16 * m >= n * n));
     }
     static bool long_rows(const Level<O, E, W>& L) { return long_rows((int64_t)L.n, (int64_t)L.m, (int64_t)L.max_deg, (int64_t)L.n_hub); }
     bool cta_eligible(const Level<O, E, W>& L) const {
@@ -861,8 +864,11 @@ struct Refiner {
     // side: 600,000-vertex levels ran 106 and 79 (mesh, 600 parts), 118 and 86
     // (1,000), 114 and 64, 119 and 66 (geometric graph).
     // Nor do levels of long rows gain above that bound (R-MAT 2^19 into 64 parts:
-    // finest level 365 and 489), and with 64-bit weights they lose from fewer
-    // entries on (R-MAT 2^19's levels of 6-8 M entries 434-604 in the graph and 590-749).
+    // finest level 365 and 489), and with 64-bit weights they and levels with hubs
+    // lose from fewer entries on (R-MAT 2^19's levels of 6-8 M entries 434-604 in
+    // the graph and 590-749, a matching hierarchy's of 6-7 M 2,007 and 3,786, 3,423
+    // and 7,524). Hubs among short rows gain otherwise: that hierarchy's levels of
+    // 517,000-556,000 vertices and 0.03-3.1 M entries 142-528 and 71-229.
     static constexpr int64_t COOP_MAX_N = (int64_t)1 << 20;
     static constexpr int64_t COOP_MAX_N_MANY = (int64_t)1 << 18;
     static constexpr int64_t COOP_MAX_M_LONG = (int64_t)1 << 22;

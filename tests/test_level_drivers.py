@@ -83,7 +83,8 @@ def test_wide_weights_and_many_parts_keep_the_persistent_loops(jet, graphs, orc,
 
 
 @pytest.mark.parametrize("n,m,max_deg,n_hub,want", [
-    (10000, 60000, 60, 0, 0), (10000, 60000, 5000, 1, 1),                          # a mesh; one hub row
+    (10000, 60000, 60, 0, 0), (10000, 60000, 5000, 1, 0),                          # a mesh; hubs among short rows
+    (10000, 139999, 5000, 1, 0), (10000, 140000, 5000, 1, 1),                      # hubs and a mean of 14
     (10000, 320000, 127, 0, 0), (10000, 320000, 128, 0, 1),                        # longest row of four times the mean
     (10000, 319999, 4000, 0, 0),                                                   # a mean below 32
     (513, 16416, 60, 0, 0), (512, 16384, 60, 0, 1), (200000, 26000000, 300, 0, 0)  # small and dense; large and dense
@@ -148,12 +149,15 @@ def test_long_rows_on_the_persistent_loops(jet, long_row_graphs, drivers, tier, 
 @pytest.mark.gpu
 @pytest.mark.parametrize("scale,degree,tier,wide,loops", [
     (18, 8, "i32", False, {"coop"}), (19, 8, "i32", False, set()), (18, 10, "i32", False, {"coop"}),
-    (18, 8, "big", True, {"coop"}), (18, 10, "big", True, set())])
+    (19, 3, "i32", False, {"coop"}), (19, 6, "i32", False, {"coop"}), (18, 8, "big", True, {"coop"}),
+    (18, 10, "big", True, set()), (19, 3, "big", True, {"coop"}), (19, 6, "big", True, set())])
 def test_large_levels_of_long_rows_stay_level_graphs(jet, graphs, scale, degree, tier, wide, loops):
     """Power-law levels above 262,144 vertices, and with 64-bit weights above
-    2^22 entries, are faster as level graphs than on the grid."""
+    2^22 entries, are faster as level graphs than on the grid; those of mostly
+    short rows only with 64-bit weights and above 2^22 entries."""
     g = graphs.rmat(scale, degree, seed=4, tier=tier, device="cuda").as_tier(tier)
-    assert (g.nnz > 1 << 22) == (degree == 10 or scale == 19)
+    assert (g.nnz > 1 << 22) == (degree == 10 or (scale, degree) in ((19, 6), (19, 8)))
+    assert int((g.row[1:] - g.row[:-1]).max()) > 4096
     if wide:
         g.val = g.val * (2 ** 31 // int(g.val.sum()) + 1)
     part = torch.randint(0, 16, (g.n,), generator=torch.Generator().manual_seed(1), dtype=torch.int32).cuda()
